@@ -515,6 +515,19 @@ int tnb_block_svd(const int64_t* rows, int64_t n_rows, const double* a, int64_t 
                   void* stream);
 
 /*
+ * The same factorisation with each sector on a thread-block cluster, a warp per column pair
+ * (rows as above, w_off unused).  Takes sectors with max(m, n) <= max_r <= 512 and
+ * min(m, n) <= max_c <= 256; tnb_block_svd_cluster_ok says whether a launch with these
+ * bounds can run on the current device (1) or not (0).  Same singular values and vectors
+ * as tnb_block_svd to rounding, in the same gauge.
+ */
+int tnb_block_svd_cluster_ok(int64_t max_r, int64_t max_c);
+int tnb_block_svd_cluster(const int64_t* rows, int64_t n_rows, const double* a, int64_t n_a,
+                          double* u, int64_t n_u, double* s, int64_t n_s, double* vt,
+                          int64_t n_vt, int32_t* info, int64_t max_r, int64_t max_c,
+                          void* stream);
+
+/*
  * The truncation decision on the device: _spectrum / _admissible / _decide of
  * ops/linalg.py:1079-1324 in one CTA.  sectors: n_sec rows of 4 int64 [count, s_off,
  * label, 0] in ascending label order, each a descending list of `count` singular values

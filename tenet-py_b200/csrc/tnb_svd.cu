@@ -145,15 +145,15 @@ block_svd_kernel(const int64_t* __restrict__ rows, int64_t n_rows, const double*
         const double cs = 1.0 / sqrt(fma(t, t, 1.0)), sn = cs * t;
         for (int64_t q = lane; q < r; q += 32) {
           const double x = wi[q], y = wj[q];
-          wi[q] = cs * x - sn * y;
-          wj[q] = sn * x + cs * y;
+          wi[q] = fma(cs, x, -__dmul_rn(sn, y));
+          wj[q] = fma(sn, x, __dmul_rn(cs, y));
         }
         double* vi = V + static_cast<int64_t>(i) * c;
         double* vj = V + static_cast<int64_t>(j) * c;
         for (int64_t q = lane; q < c; q += 32) {
           const double x = vi[q], y = vj[q];
-          vi[q] = cs * x - sn * y;
-          vj[q] = sn * x + cs * y;
+          vi[q] = fma(cs, x, -__dmul_rn(sn, y));
+          vj[q] = fma(sn, x, __dmul_rn(cs, y));
         }
         if (lane == 0) s_rotated = 1;
       }

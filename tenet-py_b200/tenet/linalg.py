@@ -115,28 +115,41 @@ class _SvdPlan:
         p = m.provider
         self.ml = ml
         self.sectors = tuple(sorted(ml.sectors))
-        smem_max = int(_lib.load().tnb_block_svd_smem_doubles())
+        lib = _lib.load()
+        smem_max = int(lib.tnb_block_svd_smem_doubles())
         rows, sec_rows, qd = [], [], []
         self.kfull = {}
         uo = so = vo = wo = 0
         smem = 0
+        # the sectors a cluster launch takes come first: all but the largest ones
+        shapes = sorted((max(ml.shape[c]), min(ml.shape[c]), c) for c in self.sectors)
+        while shapes and not lib.tnb_block_svd_cluster_ok(
+                max(x[0] for x in shapes), max(x[1] for x in shapes)):
+            shapes.pop()
+        clustered = {c for _, _, c in shapes}
+        self.n_cluster = len(shapes)
+        self.max_r = max((x[0] for x in shapes), default=0)
+        self.max_c = max((x[1] for x in shapes), default=0)
         for c in self.sectors:
             r, q = ml.shape[c]
             k = min(r, q)
             need = max(r, q) * k + k * k + 2 * k
-            if need <= smem_max:
+            if c in clustered:
+                w = -1
+            elif need <= smem_max:
                 w = -1
                 smem = max(smem, need)
             else:
                 w = wo
                 wo += need
-            rows.append((r, q, ml.base[c], uo, so, vo, w, 0))
+            rows.append((c not in clustered, (r, q, ml.base[c], uo, so, vo, w, 0)))
             sec_rows.append((k, so, c, 0))
             qd.append(float(p._qdim(c)))
             self.kfull[c] = (k, uo, so, vo)
             uo, so, vo = uo + r * k, so + k, vo + k * q
         self.n_u, self.n_s, self.n_v, self.n_w, self.smem = uo, so, vo, wo, smem
         self.total = so
+        rows = [x for _, x in sorted(rows, key=lambda x: x[0])]
         dev = _exec.device()
         i64 = dict(dtype=torch.int64, device=dev)
         self.rows = torch.tensor(rows or [(0,) * 8], **i64)
@@ -258,8 +271,15 @@ def svd_truncated_launch(t: SymmetricTensor, axes=None, *, max_bond=None, cutoff
     ns = len(plan.sectors)
     rb = plan.readback(st)
     base = rb.dev.data_ptr()
-    _lib.call("tnb_block_svd", P(plan.rows), ns, P(buf), buf.numel(), P(U), U.numel(), P(Sv),
-              Sv.numel(), P(V), V.numel(), P(W), plan.n_w, base + plan.o_info, plan.smem, st)
+    nc = plan.n_cluster
+    if nc:
+        _lib.call("tnb_block_svd_cluster", P(plan.rows), nc, P(buf), buf.numel(), P(U), U.numel(),
+                  P(Sv), Sv.numel(), P(V), V.numel(), base + plan.o_info, plan.max_r, plan.max_c,
+                  st)
+    if nc < ns:
+        _lib.call("tnb_block_svd", P(plan.rows) + 64 * nc, ns - nc, P(buf), buf.numel(), P(U),
+                  U.numel(), P(Sv), Sv.numel(), P(V), V.numel(), P(W), plan.n_w,
+                  base + plan.o_info + 4 * nc, plan.smem, st)
     _lib.call("tnb_truncate_decide", P(plan.sec_rows), P(plan.qdim), ns, P(Sv), Sv.numel(),
               -1.0 if cutoff is None else float(cutoff), _MODES[cutoff_mode],
               -1.0 if max_bond is None else float(max_bond), 0 if budget == "dense" else 1,
