@@ -243,6 +243,137 @@ block_svd_kernel(const int64_t* __restrict__ rows, int64_t n_rows, const double*
   if (tid == 0) info[b] = converged ? 0 : sweep;
 }
 
+// The decision of a spectrum of T <= kDecideStaged values, staged in shared memory.  The
+// reference's sums run one value after another, so each is a chain of T dependent additions;
+// what varies with the decision is only where a chain is read.  The running sums -- from the
+// end for the cutoff, from the front for the budget and the kept weight, and the two totals --
+// are therefore written out by one thread each, all at once, and every walk becomes a count
+// over a monotone sequence.  (One thread walking the values in global memory took 112 us for
+// 512 values of 10 sectors.)
+constexpr int kDecideStaged = 1024;
+
+struct DecideSmem {
+  double x[kDecideStaged];        // the sectors' lists, then the values in global order
+  double q[kDecideStaged];        // their quantum dimensions
+  double drop[kDecideStaged];     // sum of weights from the end down to e
+  double dense[kDecideStaged];    // sum of qdim up to e
+  double kept[kDecideStaged];     // sum of qdim sigma^2 up to e
+  double total, total2;
+  int keep[256];
+};
+
+__device__ void decide_staged(const int64_t* sectors, const double* qdim, int n_sec,
+                              const double* s, const int64_t* begin, int T, double cutoff,
+                              int mode, double max_bond, int budget, int64_t* keep,
+                              double* sorted_s, int32_t* sorted_c, double* stats) {
+  __shared__ DecideSmem sm;
+  const int tid = threadIdx.x;
+  const int e = tid;  // kDecideThreads >= kDecideStaged: a thread per value
+  int k = 0;
+  if (e < T) {
+    while (k + 1 < n_sec && begin[k + 1] <= e) ++k;
+    sm.x[e] = s[sectors[k * kSectorRow + 1] + (e - begin[k])];
+  }
+  if (tid < 256) sm.keep[tid] = 0;
+  __syncthreads();
+  // global rank of (sigma, sector, index), as in decide_kernel
+  int rank = -1;
+  double v = 0.0;
+  if (e < T) {
+    v = sm.x[e];
+    rank = e - static_cast<int>(begin[k]);
+    for (int o = 0; o < n_sec; ++o) {
+      if (o == k) continue;
+      const double* so = sm.x + begin[o];
+      int lo = 0, hi = static_cast<int>(begin[o + 1] - begin[o]);
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (o < k ? so[mid] >= v : so[mid] > v) lo = mid + 1; else hi = mid;
+      }
+      rank += lo;
+    }
+    sorted_c[e] = -1;
+  }
+  __syncthreads();
+  int* const owner = reinterpret_cast<int*>(sm.kept);  // until the running sums are formed
+  for (int i = tid; i < T; i += kDecideThreads) owner[i] = -1;
+  __syncthreads();
+  if (e < T) {
+    sm.x[rank] = v;
+    owner[rank] = k;
+    sm.q[rank] = qdim[k];
+    sorted_s[rank] = v;
+  }
+  __syncthreads();
+  const int own = e < T ? owner[e] : 0;
+  if (e < T) sorted_c[e] = own;
+  if (tid < n_sec) keep[tid] = 0;
+  if (__syncthreads_or(own < 0)) {  // a NaN breaks the order
+    if (tid == 0) raise_bounds();
+    if (tid < 8) stats[tid] = 0.0;
+    return;
+  }
+  const bool sums = cutoff >= 0.0 && mode > 1, sq = mode == 2 || mode == 3;
+  if (tid == 0) {
+    double t = 0.0;
+    const int end = sums ? T : 0;
+#pragma unroll 8
+    for (int i = 0; i < end; ++i) t = fma(sm.q[i], sq ? sm.x[i] * sm.x[i] : sm.x[i], t);
+    sm.total = t;
+  } else if (tid == 32) {
+    double d = 0.0;
+#pragma unroll 8
+    for (int i = sums ? T - 1 : -1; i >= 0; --i) {
+      d = fma(sm.q[i], sq ? sm.x[i] * sm.x[i] : sm.x[i], d);
+      sm.drop[i] = d;
+    }
+  } else if (tid == 64) {
+    double d = 0.0;
+#pragma unroll 8
+    for (int i = 0; i < T; ++i) {
+      d += sm.q[i];
+      sm.dense[i] = d;
+    }
+  } else if (tid == 96) {
+    double d = 0.0;
+#pragma unroll 8
+    for (int i = 0; i < T; ++i) {
+      d = fma(sm.q[i] * sm.x[i], sm.x[i], d);
+      sm.kept[i] = d;
+    }
+    sm.total2 = d;  // the kept weight of everything is the total: the same chain
+  }
+  __syncthreads();
+  // admissible values, and those within the budget
+  bool above = e < T;
+  if (cutoff >= 0.0 && e < T) {
+    if (mode <= 1)
+      above = sm.x[e] > (mode == 0 ? cutoff : cutoff * sm.x[0]);
+    else
+      above = sm.drop[e] >= ((mode == 3 || mode == 5) ? cutoff * sm.total : cutoff);
+  }
+  const int adm = __syncthreads_count(above);
+  const double used = e < T ? (budget == 0 ? sm.dense[e] : static_cast<double>(e + 1)) : 0.0;
+  const int fits = __syncthreads_count(e < T && !(max_bond >= 0.0 && used > max_bond));
+  const int n_kept = adm < fits ? adm : fits;
+  if (e < n_kept) atomicAdd(&sm.keep[own], 1);
+  __syncthreads();
+  if (tid < n_sec) keep[tid] = sm.keep[tid];
+  if (tid == 0) {
+    double disc = 0.0;
+#pragma unroll 8
+    for (int i = n_kept; i < T; ++i) disc = fma(sm.q[i] * sm.x[i], sm.x[i], disc);
+    stats[0] = static_cast<double>(n_kept);
+    stats[1] = n_kept ? sm.dense[n_kept - 1] : 0.0;
+    stats[2] = disc;
+    stats[3] = sm.total2;
+    stats[4] = n_kept ? sm.kept[n_kept - 1] : 0.0;
+    stats[5] = static_cast<double>(adm);
+    stats[6] = static_cast<double>(T);
+    stats[7] = 0.0;
+  }
+}
+
 // One CTA.  sectors: rows of [count, s_off, label, 0] sorted by label; qdim per sector.
 // mode: 0 abs, 1 rel, 2 sum2, 3 rsum2, 4 sum1, 5 rsum1; cutoff < 0: no cutoff;
 // max_bond < 0: no budget; budget: 0 dense (cost qdim), 1 reduced (cost 1).
@@ -275,6 +406,11 @@ decide_kernel(const int64_t* __restrict__ sectors, const double* __restrict__ qd
   __syncthreads();
   const int64_t T = s_begin[n_sec];
   if (T < 0) return;
+  if (T <= kDecideStaged) {
+    decide_staged(sectors, qdim, static_cast<int>(n_sec), s, s_begin, static_cast<int>(T), cutoff,
+                  mode, max_bond, budget, keep, sorted_s, sorted_c, stats);
+    return;
+  }
   // global rank of every (sigma, sector, index)
   for (int64_t e = tid; e < T; e += kDecideThreads) sorted_c[e] = -1;
   __syncthreads();

@@ -8,7 +8,8 @@ import pytest
 import torch
 
 from test_gpu_svd import _check, _svd_batch
-from tenet import _exec, _lib
+from tenet import _exec, _lib, linalg
+from tenet.symmetry import SU2
 
 pytestmark = pytest.mark.gpu
 P = _exec.ptr
@@ -88,3 +89,50 @@ def test_cluster_svd_refuses_what_it_cannot_hold():
     assert lib.tnb_block_svd_cluster_ok(4, 8) == 0
     assert lib.tnb_block_svd_cluster(None, 1, None, 0, None, 0, None, 0, None, 0, None, 600, 10,
                                      None) == 1
+
+
+@pytest.mark.parametrize("total", [1, 31, 1023, 1024, 1025, 2500])
+@pytest.mark.parametrize("mode,cutoff", [("rsum2", 1e-6), ("sum1", 1e-2), ("rel", 1e-3),
+                                         ("rsum2", None)])
+def test_decision_staged_and_streamed(total, mode, cutoff):
+    """Spectra on both sides of the staged decision's limit (1024 values) against the host
+    rule: kept counts, order and sums (sums to 1e-12: a few thousand roundings)."""
+    rng = np.random.default_rng(total)
+    labels = [0, 2, 4, 6, 8][:min(5, total)]
+    cuts = np.sort(rng.choice(np.arange(1, total), size=len(labels) - 1, replace=False)) \
+        if len(labels) > 1 else np.zeros(0, int)
+    sizes = np.diff(np.concatenate([[0], cuts, [total]]))
+    spectra = [np.sort(10.0 ** -rng.integers(0, 400, n).astype(float) ** 0.25)[::-1]
+               for n in sizes]
+    spectrum = sorted(((float(x), c, i) for c, sp in zip(labels, spectra)
+                       for i, x in enumerate(sp)), key=lambda e: (-e[0], e[1], e[2]))
+    offs = np.concatenate([[0], np.cumsum(sizes)])
+    i64 = dict(dtype=torch.int64, device="cuda")
+    s = torch.tensor(np.concatenate(spectra), device="cuda")
+    sec = torch.tensor([(n, offs[k], c, 0) for k, (c, n) in enumerate(zip(labels, sizes))], **i64)
+    qd = torch.tensor([c + 1.0 for c in labels], dtype=torch.float64, device="cuda")
+    for max_bond in (None, 1, total, 3 * total) if cutoff is not None else (1, total):
+        keep = torch.full((len(labels),), 9, **i64)
+        ss = torch.zeros(total, dtype=torch.float64, device="cuda")
+        sc = torch.zeros(total, dtype=torch.int32, device="cuda")
+        st = torch.zeros(8, dtype=torch.float64, device="cuda")
+        for budget in ("dense", "reduced"):
+            try:
+                want = linalg.decide(spectrum, SU2, max_bond, cutoff, mode, budget=budget)
+            except ValueError:  # nothing kept
+                want = None
+            _lib.call("tnb_truncate_decide", P(sec), P(qd), len(labels), P(s), total,
+                      -1.0 if cutoff is None else cutoff, linalg._MODES[mode],
+                      -1.0 if max_bond is None else float(max_bond), int(budget == "reduced"),
+                      P(keep), P(ss), P(sc), P(st), _exec.stream_ptr())
+            torch.cuda.synchronize()
+            stats = st.cpu().numpy()
+            got = {c: int(k) for c, k in zip(labels, keep.cpu().numpy()) if k}
+            assert got == ({} if want is None else want.keep)
+            order = [(float(x), labels[k]) for x, k in zip(ss.cpu().numpy(), sc.cpu().numpy())]
+            assert order == [(x, c) for x, c, _ in spectrum]
+            if want is not None:
+                assert stats[0] == want.reduced_dim and stats[1] == want.dense_dim
+                assert stats[2] == pytest.approx(want.discarded_weight, rel=1e-12, abs=1e-300)
+                assert stats[3] == pytest.approx(sum(SU2._qdim(c) * x * x for x, c, _ in spectrum),
+                                                 rel=1e-12)
