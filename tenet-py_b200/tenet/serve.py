@@ -255,7 +255,11 @@ class ProcessServer:
         self.pool = ProcessPoolExecutor(
             max_workers=workers, mp_context=multiprocessing.get_context("spawn"),
             initializer=_worker_init, initargs=(precision, ncv, cutoff, tc_min_flops))
-        self.pids = set(self.pool.map(_worker_ready, range(2 * workers)))
+        # until every worker has answered: one that is a second slower to start would
+        # otherwise leave its share of the first round to the others
+        self.pids, end = set(), time.monotonic() + 120.0
+        while len(self.pids) < workers and time.monotonic() < end:
+            self.pids |= set(self.pool.map(_worker_ready, range(2 * workers)))
         self.peak_active = 0
 
     def close(self) -> None:
