@@ -114,6 +114,30 @@ int tnb_block_gather_direct(const int64_t* chunk_rows, int64_t total_chunks,
                             void* stream);
 
 /*
+ * The same block maps from warp items: the table as one row of `width` int32 words (32, or
+ * 64 with up to six further terms inline) per item, an item being at most
+ * TNB_ITEM_MAX_ELEMS consecutive elements of a segment (rank <= 4, offsets within a segment
+ * below 2^31).  Words: [0,1] destination offset, [2,3] first term's source, [4,5] its
+ * coefficient (64-bit values, low word first), [6] first and [7] past-the-last term, [8]
+ * first element, [9] elements, [10] rank | buffer pair << 8 | division shifts of extents
+ * 1..3 at bits 16, 21, 26, [11] first term's leading dimension, [12..15] extents, [16..18]
+ * division constants of extents 1..3, [20..23] destination, [24..27] row and [28..31]
+ * column strides, [32 + 5 i ..] term 1 + i: source, coefficient, leading dimension.
+ * tnb_plan_gather_items builds the rows on the host (rows null: only counts them) and
+ * returns their number, -1 for a table that does not fit, -2 for bad arguments.
+ */
+#define TNB_ITEM_MAX_ELEMS 256
+int64_t tnb_plan_gather_items(int64_t n_seg, const int64_t* segs, const int64_t* term_src,
+                              const double* term_coeff, const int64_t* term_ld, int64_t n_term,
+                              int64_t max_elems, int32_t width, int32_t* rows, int64_t cap);
+int tnb_block_gather_items(const int32_t* item_rows, int32_t width, int64_t n_items,
+                           const int64_t* term_src, const double* term_coeff,
+                           const int64_t* term_ld, int64_t n_term, const double* src0,
+                           int64_t n_src0, double* dst0, int64_t n_dst0, const double* src1,
+                           int64_t n_src1, double* dst1, int64_t n_dst1, void* stream);
+
+
+/*
  * Block gather whose source is a product with a short K, never materialised: the source
  * is C = A * B over the grouped-GEMM table prod_table (n_prod rows in the TNB_GEMM_WIDTH
  * layout below, K at most 4).  The segment rows are those of tnb_block_gather, with one
@@ -375,6 +399,11 @@ int tnb_seq_add_gather_direct(tnb_seq* s, const int64_t* chunk_rows, int64_t tot
                               const int64_t* term_ld, int64_t n_term, const double* src0,
                               int64_t n_src0, double* dst0, int64_t n_dst0, const double* src1,
                               int64_t n_src1, double* dst1, int64_t n_dst1);
+int tnb_seq_add_gather_items(tnb_seq* s, const int32_t* item_rows, int32_t width,
+                             int64_t n_items, const int64_t* term_src, const double* term_coeff,
+                             const int64_t* term_ld, int64_t n_term, const double* src0,
+                             int64_t n_src0, double* dst0, int64_t n_dst0, const double* src1,
+                             int64_t n_src1, double* dst1, int64_t n_dst1);
 int tnb_seq_add_gemm(tnb_seq* s, const int64_t* gemm_table, int64_t n_gemm,
                      const int32_t* tile_map, int64_t total_tiles, int32_t tile_kind,
                      const double* a, int64_t n_a, const double* b, int64_t n_b, double* c,

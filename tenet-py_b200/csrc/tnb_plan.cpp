@@ -4,10 +4,12 @@
 //                         destination stride, extent-1 dims dropped, contiguous dims merged);
 //   tnb_plan_gather_table a block map's whole gather table: terms grouped by destination
 //                         block, one row per block with terms, then zero-writing rows;
+//   tnb_plan_gather_items the table as one row per warp item (tnb_block_gather_items);
 //   tnb_plan_compose      the sparse product of two block maps (ops/repartition.py:298-316).
 #include <stdint.h>
 
 #include <algorithm>
+#include <cstring>
 #include <numeric>
 #include <unordered_map>
 #include <vector>
@@ -213,4 +215,104 @@ extern "C" int64_t tnb_plan_compose(int64_t n_a, const double* a, int64_t n_b, c
     }
   }
   return n_out;
+}
+
+extern "C" int64_t tnb_plan_gather_items(int64_t n_seg, const int64_t* segs,
+                                         const int64_t* term_src, const double* term_coeff,
+                                         const int64_t* term_ld, int64_t n_term,
+                                         int64_t max_elems, int32_t width, int32_t* rows,
+                                         int64_t cap) {
+  if (n_seg < 0 || n_term < 0 || n_term > INT32_MAX || (n_seg && !segs) ||
+      (n_term && (!term_src || !term_coeff || !term_ld)) || max_elems < 32 ||
+      max_elems > TNB_ITEM_MAX_ELEMS || max_elems % 32 || (width != 32 && width != 64) || cap < 0)
+    return -2;
+  constexpr int64_t kLim = INT32_MAX;
+  int64_t count = 0;
+  for (int64_t g = 0; g < n_seg; ++g) {
+    const int64_t* s = segs + g * kSegW;
+    const int64_t size = s[1], rank = s[2], t0 = s[3], t1 = s[4];
+    if (t0 < 0 || t1 < t0 || t1 > n_term) return -2;
+    if (rank < 1 || rank > 4 || size < 0 || size > kLim) return -1;
+    if (size == 0) continue;
+    // every offset within the segment fits 32 bits, for each of its terms
+    int64_t d_span = 0, total = 1;
+    for (int64_t d = 0; d < rank; ++d) {
+      const int64_t e = s[8 + d];
+      if (e < 1 || e > kLim || (d > 0 && e < 2)) return -1;
+      total *= e;
+      if (total > kLim) return -1;
+      for (int k = 16; k <= 32; k += 8)
+        if (s[k + d] > kLim || s[k + d] < -kLim) return -1;
+      d_span += (e - 1) * std::abs(s[16 + d]);
+    }
+    if (total != size || d_span > kLim) return -1;
+    for (int64_t t = t0; t < t1; ++t) {
+      const int64_t ld = term_ld[t];
+      if (ld > kLim || ld < -kLim) return -1;
+      int64_t span = 0;
+      for (int64_t d = 0; d < rank; ++d) {
+        const __int128 x = static_cast<__int128>(s[8 + d] - 1) *
+                           (static_cast<__int128>(ld < 0 ? -ld : ld) * std::abs(s[24 + d]) +
+                            std::abs(s[32 + d]));
+        if (x > kLim) return -1;
+        span += static_cast<int64_t>(x);
+      }
+      // the strides themselves too: a one-term item multiplies by ld r + c
+      for (int64_t d = 0; d < rank; ++d)
+        if (static_cast<__int128>(ld < 0 ? -ld : ld) * std::abs(s[24 + d]) + std::abs(s[32 + d]) >
+            kLim)
+          return -1;
+      if (span > kLim) return -1;
+    }
+    const int64_t parts = (size + max_elems - 1) / max_elems;
+    const int64_t per = ((size + parts - 1) / parts + 31) / 32 * 32;  // even parts, whole warps
+    const int64_t n_items = (size + per - 1) / per;
+    if (rows == nullptr) {
+      count += n_items;
+      continue;
+    }
+    if (count + n_items > cap) return -2;
+    int32_t head[64] = {0};
+    auto put64 = [&](int at, const void* v) { std::memcpy(head + at, v, 8); };
+    put64(0, s);
+    if (t1 > t0) {
+      put64(2, term_src + t0);
+      put64(4, term_coeff + t0);
+      head[11] = static_cast<int32_t>(term_ld[t0]);
+    }
+    head[6] = static_cast<int32_t>(t0);
+    head[7] = static_cast<int32_t>(t1);
+    int64_t meta = rank | (s[5] != 0 ? 256 : 0);
+    for (int64_t d = 0; d < rank; ++d) {
+      const int64_t e = s[8 + d];
+      head[12 + d] = static_cast<int32_t>(e);
+      head[20 + d] = static_cast<int32_t>(s[16 + d]);
+      head[24 + d] = static_cast<int32_t>(s[24 + d]);
+      head[28 + d] = static_cast<int32_t>(s[32 + d]);
+      if (d > 0) {  // floor(q / e) = (q mul) >> (31 + l) for q < 2^31, l = ceil(log2 e)
+        int l = 0;
+        while ((int64_t{1} << l) < e) ++l;
+        const uint64_t mul = ((uint64_t{1} << (31 + l)) + static_cast<uint64_t>(e) - 1) /
+                             static_cast<uint64_t>(e);
+        head[15 + d] = static_cast<int32_t>(static_cast<uint32_t>(mul));
+        meta |= static_cast<int64_t>(l - 1) << (11 + 5 * d);
+      }
+    }
+    head[10] = static_cast<int32_t>(static_cast<uint32_t>(meta));
+    if (width == 64)
+      for (int64_t i = 1; i <= 6 && t0 + i < t1; ++i) {
+        const int at = static_cast<int>(32 + 5 * (i - 1));
+        put64(at, term_src + t0 + i);
+        put64(at + 2, term_coeff + t0 + i);
+        head[at + 4] = static_cast<int32_t>(term_ld[t0 + i]);
+      }
+    for (int64_t i = 0; i < n_items; ++i) {
+      int32_t* r = rows + (count + i) * width;
+      std::memcpy(r, head, sizeof(int32_t) * static_cast<size_t>(width));
+      r[8] = static_cast<int32_t>(i * per);
+      r[9] = static_cast<int32_t>(std::min(per, size - i * per));
+    }
+    count += n_items;
+  }
+  return count;
 }

@@ -35,6 +35,7 @@ constexpr int32_t kOpGatherProduct = 4;
 constexpr int32_t kOpCluster = 5;
 constexpr int32_t kOpGemmGatherA = 6;
 constexpr int32_t kOpGatherDirect = 7;
+constexpr int32_t kOpGatherItems = 8;
 
 struct FStage {
   int32_t code;
@@ -219,6 +220,7 @@ constexpr int kGemmBufs[] = {5, 7, 9};          // a, b, c
 constexpr int kGatherProductBufs[] = {11, 13, 15};  // a, b, dst
 constexpr int kGemmGatherABufs[] = {9, 11, 13};     // src, b, c
 constexpr int kGatherDirectBufs[] = {6, 8, 10, 12};  // src0, dst0, src1, dst1
+constexpr int kGatherItemsBufs[] = {7, 9, 11, 13};   // src0, dst0, src1, dst1
 
 inline void* as_ptr(int64_t w) { return reinterpret_cast<void*>(static_cast<intptr_t>(w)); }
 inline int64_t as_word(const void* p) { return static_cast<int64_t>(reinterpret_cast<intptr_t>(p)); }
@@ -270,6 +272,15 @@ int replay(const tnb_seq* s, int32_t n_patch, const void* const* from, void* con
           static_cast<const double*>(as_ptr(w[6])), w[7], static_cast<double*>(as_ptr(w[8])),
           w[9], static_cast<const double*>(as_ptr(w[10])), w[11],
           static_cast<double*>(as_ptr(w[12])), w[13], stream);
+    } else if (op.code == kOpGatherItems) {
+      for (int k : kGatherItemsBufs) w[k] = patched(w[k], n_patch, from, to);
+      rc = tnb_block_gather_items(
+          static_cast<const int32_t*>(as_ptr(w[0])), static_cast<int32_t>(w[1]), w[2],
+          static_cast<const int64_t*>(as_ptr(w[3])), static_cast<const double*>(as_ptr(w[4])),
+          static_cast<const int64_t*>(as_ptr(w[5])), w[6],
+          static_cast<const double*>(as_ptr(w[7])), w[8], static_cast<double*>(as_ptr(w[9])),
+          w[10], static_cast<const double*>(as_ptr(w[11])), w[12],
+          static_cast<double*>(as_ptr(w[13])), w[14], stream);
     } else if (op.code == kOpGemmGatherA) {
       for (int k : kGemmGatherABufs) w[k] = patched(w[k], n_patch, from, to);
       rc = tnb_grouped_gemm_gather_a(
@@ -406,6 +417,24 @@ extern "C" int tnb_seq_add_gather_direct(tnb_seq* s, const int64_t* chunk_rows,
   using tnb::as_word;
   tnb_seq::Op op{tnb::kOpGatherDirect,
                  {as_word(chunk_rows), total_chunks, as_word(term_src), as_word(term_coeff),
+                  as_word(term_ld), n_term, as_word(src0), n_src0, as_word(dst0), n_dst0,
+                  as_word(src1), n_src1, as_word(dst1), n_dst1}};
+  s->ops.push_back(op);
+  return TNB_OK;
+}
+
+extern "C" int tnb_seq_add_gather_items(tnb_seq* s, const int32_t* item_rows, int32_t width,
+                                        int64_t n_items, const int64_t* term_src,
+                                        const double* term_coeff, const int64_t* term_ld,
+                                        int64_t n_term, const double* src0, int64_t n_src0,
+                                        double* dst0, int64_t n_dst0, const double* src1,
+                                        int64_t n_src1, double* dst1, int64_t n_dst1) {
+  TNB_REQUIRE(s != nullptr, "tnb_seq_add_gather_items: null sequence");
+  TNB_REQUIRE(n_items >= 0 && n_term >= 0 && (width == 32 || width == 64),
+              "tnb_seq_add_gather_items: negative size or bad row width");
+  using tnb::as_word;
+  tnb_seq::Op op{tnb::kOpGatherItems,
+                 {as_word(item_rows), width, n_items, as_word(term_src), as_word(term_coeff),
                   as_word(term_ld), n_term, as_word(src0), n_src0, as_word(dst0), n_dst0,
                   as_word(src1), n_src1, as_word(dst1), n_dst1}};
   s->ops.push_back(op);

@@ -205,22 +205,24 @@ class _UploadSlice:
         return self.up.ready()[self.lo:self.hi]
 
 
-def upload_together(tables) -> None:
-    """One upload (one staging copy, one device buffer, one event) for the arrays of every
-    table in ``tables`` not yet on the device, instead of one each at its first run."""
-    todo, arrays, spans = [], [], []
+def upload_together(tables, recorded: bool = False) -> None:
+    """One upload (one staging copy, one device buffer, one event) for the arrays that every
+    table in ``tables`` will read and that are not yet on the device, instead of one each
+    at its first run.  ``recorded``: the tables are about to be recorded into a sequence."""
+    todo, arrays = [], []
     for t in tables:
-        if t is None or getattr(t, "_dev", 1) is not None:
+        if t is None:
             continue
-        arrs = t.host_arrays()
-        todo.append(t)
-        spans.append((len(arrays), len(arrays) + len(arrs)))
+        attr, arrs = t.pending_upload(recorded)
+        if attr is None:
+            continue
+        todo.append((t, attr, len(arrays), len(arrays) + len(arrs)))
         arrays.extend(arrs)
     if not todo:
         return
     up = Uploaded(arrays)
-    for t, (lo, hi) in zip(todo, spans):
-        t._dev = _UploadSlice(up, lo, hi)
+    for t, attr, lo, hi in todo:
+        setattr(t, attr, _UploadSlice(up, lo, hi))
 
 
 class Uploaded:
@@ -403,6 +405,9 @@ class GatherTable:
         self.chunk_map = np.repeat(np.arange(len(seg), dtype=np.int32), per)
         self._dev = None
         self._ddev = None
+        self._items = None  # (width, items, rows) or False: built by item_rows()
+        self._idev = None
+        self._choice = self._head = None
 
     @property
     def bytes_moved(self) -> int:
@@ -446,10 +451,77 @@ class GatherTable:
             self._ddev = Uploaded((self.chunk_rows(), self.tsrc, self.tcf, self.tld))
         return self._ddev.ready()
 
+    def item_rows(self):
+        """``(row width, items, rows)`` of the table as warp items
+        (``tnb_block_gather_items``), or None when a segment's rank or offsets do not fit
+        one."""
+        if self._items is None:
+            lib, seg = _lib.load(), np.ascontiguousarray(self.seg, dtype=np.int64)
+            width = 64 if self.n_seg and int((seg[:, 4] - seg[:, 3]).max()) > 1 else 32
+            cap = item_size(self.elems)
+            args = (self.n_seg, seg.ctypes.data, self.tsrc.ctypes.data, self.tcf.ctypes.data,
+                    self.tld.ctypes.data, self.n_term, cap, width)
+            n = int(lib.tnb_plan_gather_items(*args, None, 0))
+            if n < -1:
+                raise ValueError("item_rows: a malformed gather table")
+            self._items = False
+            if n > 0:
+                rows = np.empty((n, width), dtype=np.int32)
+                if int(lib.tnb_plan_gather_items(*args, rows.ctypes.data, n)) != n:
+                    raise ValueError("item_rows: a malformed gather table")
+                self._items = (width, n, rows)
+        return self._items or None
+
+    def takes_items(self, recorded: bool) -> bool:
+        """Whether a run (or a recording) of this table goes through its warp items."""
+        if not (DIRECT_GATHER and (CHAIN_ITEMS and not _STANDARD[0] if recorded
+                                   else self.chunks >= DIRECT_MIN_CHUNKS)):
+            return False
+        return self.item_rows() is not None
+
+    def pending_upload(self, recorded: bool) -> tuple:
+        """``(attribute, arrays)`` of the device copy a run will read, ``(None, ())`` when
+        it is already there."""
+        if type(self) is GatherTable and self.takes_items(recorded):
+            if self._idev is not None:
+                return None, ()
+            return "_idev", (self.item_rows()[2], self.tsrc, self.tcf, self.tld)
+        return ("_dev", self.host_arrays()) if self._dev is None else (None, ())
+
+    def item_arrays(self):
+        if self._idev is None:
+            self._idev = Uploaded((self.item_rows()[2], self.tsrc, self.tcf, self.tld))
+        return self._idev.ready()
+
     def run(self, src0, dst0, src1=None, dst1=None) -> None:
         if self.n_seg == 0:
             return
         rec = recording()
+        if rec is None:
+            c = self._choice  # whether launches take the items, under the flags it was made for
+            if c is None or c[0] is not DIRECT_GATHER or c[1] != DIRECT_MIN_CHUNKS:
+                c = self._choice = (DIRECT_GATHER, DIRECT_MIN_CHUNKS, self.takes_items(False))
+            items = c[2]
+        else:
+            items = not CHAIN_DIRECT_GATHER and self.takes_items(True)
+        if items:
+            if self._head is None:  # the table's share of the call's arguments
+                rows, tsrc, tcf, tld = self.item_arrays()
+                self._head = (ptr(rows), *self._items[:2], ptr(tsrc), ptr(tcf), ptr(tld),
+                              self.n_term)
+            else:
+                self._idev.ready()  # (a run on another stream than the upload's)
+            args = (*self._head, ptr(src0), src0.numel(), ptr(dst0), dst0.numel(),
+                    ptr(src1), 0 if src1 is None else src1.numel(),
+                    ptr(dst1), 0 if dst1 is None else dst1.numel())
+            if rec is not None:
+                _lib.call("tnb_seq_add_gather_items", rec.handle, *args)
+                return
+            mark = _LOG.begin() if _LOG is not None else None
+            _lib.call("tnb_block_gather_items", *args, stream_ptr())
+            if _LOG is not None:
+                _LOG.end("block_gather", mark, self.bytes_moved)
+            return
         if rec is not None and CHAIN_DIRECT_GATHER and not _STANDARD[0] and self.direct_ok:
             crows, tsrc, tcf, tld = self.direct_arrays()
             _lib.call("tnb_seq_add_gather_direct", rec.handle, ptr(crows), self.chunks,
@@ -485,11 +557,17 @@ class GatherTable:
             _LOG.end("block_gather", mark, self.bytes_moved)
 
 
-#: run gathers of at least DIRECT_MIN_CHUNKS chunks (more than two waves of resident
-#: CTAs, where each CTA's table loads are not hidden behind another kernel) from their
-#: per-chunk rows (``tnb_block_gather_direct``): one round of table loads per CTA
+#: run gathers of at least DIRECT_MIN_CHUNKS chunks from warp items
+#: (``tnb_block_gather_items``) where the table fits them (rank <= 4, 32-bit offsets within
+#: a segment), else from per-chunk rows (``tnb_block_gather_direct``).  Items win at every
+#: size: config-3's batched gathers 5.5 TB/s against 1.6 (439 against 1446 us in all), a
+#: 974-element one 1.3 against 1.8 us
 DIRECT_GATHER = True
-DIRECT_MIN_CHUNKS = 2 * 3 * N_SM + 1
+DIRECT_MIN_CHUNKS = 0
+#: record the gathers of compiled chains as warp items too (a matvec on 256 multiplets 36.7
+#: against 39.0 us, with a cold L2 41.0 against 45.0; on the L = 64 mid bond 14.4-16.4 against
+#: 16.4, cold 20.4 against 22.4)
+CHAIN_ITEMS = True
 DIRECT_MAX_RANK = 4
 #: record the gathers of compiled chains (a matvec's recorded sequence) in the per-chunk-row
 #: form whatever their size.  Off by default: the same bits, but a one-wave gather's table
@@ -530,6 +608,18 @@ def chunk_size(sizes, ctas_per_sm: int = GATHER_CTAS_PER_SM) -> int:
         if int(((sizes + ce - 1) // ce).sum()) >= wave:
             return ce
     return CHUNK // 4
+
+
+def item_size(elems: int) -> int:
+    """Elements per warp item of a gather of ``elems`` elements: 256, or 128 and 64 for
+    tables that would otherwise leave SMs without a warp.  Smaller items measured slower:
+    more CTAs start for the same bytes (a compiled matvec on 256 multiplets, whose larger
+    gather has 240,000 elements: 36.7 us with 256, 38.4 with 128, 43.7 with 64; at 974 and
+    4,140 elements 64 and 32 are equal)."""
+    size = 256
+    while size > 64 and elems < size * N_SM:
+        size //= 2
+    return size
 
 
 def _chunked(seg: np.ndarray, ctas_per_sm: int = GATHER_CTAS_PER_SM) -> np.ndarray:
@@ -712,6 +802,9 @@ class GemmTable:
     def host_arrays(self) -> tuple:
         return (self.table, self.tile_map)
 
+    def pending_upload(self, recorded: bool) -> tuple:
+        return ("_dev", self.host_arrays()) if self._dev is None else (None, ())
+
     def device_tables(self):
         """(table, tile_map) on the current device, uploaded on first use."""
         if self._dev is None:
@@ -862,6 +955,9 @@ class GatherAGemm:
 
     def host_arrays(self) -> tuple:
         return (self.table, self.tile_map, self.a_ptr, self.a_src, self.a_cf)
+
+    def pending_upload(self, recorded: bool) -> tuple:
+        return ("_dev", self.host_arrays()) if self._dev is None else (None, ())
 
     def device_tables(self):
         if self._dev is None:

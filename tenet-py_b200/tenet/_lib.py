@@ -23,6 +23,11 @@ SIGNATURES = {
                                 _i64, _vp, _i64, _vp, _i64, _vp]),
     "tnb_block_gather_direct": (_i32, [_vp, _i64, _vp, _vp, _vp, _i64, _vp, _i64, _vp, _i64,
                                        _vp, _i64, _vp, _i64, _vp]),
+    "tnb_block_gather_items": (_i32, [_vp, _i32, _i64, _vp, _vp, _vp, _i64, _vp, _i64, _vp,
+                                      _i64, _vp, _i64, _vp, _i64, _vp]),
+    "tnb_seq_add_gather_items": (_i32, [_vp, _vp, _i32, _i64, _vp, _vp, _vp, _i64, _vp, _i64,
+                                        _vp, _i64, _vp, _i64, _vp, _i64]),
+    "tnb_plan_gather_items": (_i64, [_i64, _vp, _vp, _vp, _vp, _i64, _i64, _i32, _vp, _i64]),
     "tnb_copy_f64": (_i32, [_i64, _vp, _vp, _vp]),
     "tnb_mapped_address": (_i32, [_vp, ctypes.POINTER(_vp)]),
     "tnb_block_gather_product": (_i32, [_vp, _i64, _vp, _i64, _vp, _vp, _vp, _vp, _i64, _vp,
@@ -117,8 +122,14 @@ def load():
     return lib
 
 
+_functions: dict = {}  # bound entry points by name
+
+
 def call(name: str, *args) -> None:
-    status = getattr(load(), name)(*args)
+    fn = _functions.get(name)
+    if fn is None:
+        fn = _functions[name] = getattr(load(), name)
+    status = fn(*args)
     if status != 0:
         msg = load().tnb_last_error().decode(errors="replace")
         raise TenetCudaError(f"{name} failed with status {status}: {msg}")

@@ -333,7 +333,7 @@ class ChainProgram:
         _exec.upload_together([t for lk in self.links
                                for t in ((lk.ga, lk.b_gather) if lk.ga is not None else
                                          (lk.a_gather, lk.b_gather, *lk.gemm.parts))]
-                              + [self.out_gather])
+                              + [self.out_gather], recorded=True)
         for lk in self.links:  # split-K scratch of this program's own
             lk.gemm = lk.gemm.private()
         self.a_bufs = [torch.empty(max(1, 0 if lk.ga is not None else lk.a_size), **f64)
@@ -348,39 +348,46 @@ class ChainProgram:
         self.seq = _exec.Seq()
         with self.seq:
             self._run_tables(self.x_slot, self.y_slot)
-        # the one-launch forms fuse a chunk-map recording of the same stages
-        std = self.seq
-        if _exec.CHAIN_DIRECT_GATHER:
-            std = _exec.Seq()
-            with _exec.standard_gathers(), std:
-                self._run_tables(self.x_slot, self.y_slot)
-        self._std_seq = std
-        # the same stages as one persistent launch, when they all fuse (no tensor-core
-        # stage, no product-source gather, at most the kernel's stage count)
+        self._std_seq = self._fused = None
         self.cluster = None
         if getattr(self, "compact", False) and _exec.CLUSTER and \
-                0 < len(std) <= FUSED_MAX_STAGES:
+                0 < len(self.seq) <= FUSED_MAX_STAGES:
             import ctypes
 
             from tenet import _lib
 
             cl, ctas = _exec.Seq(), ctypes.c_int32(0)
-            _lib.call("tnb_seq_fuse_cluster", std.handle, self.x_slot.data_ptr(),
+            _lib.call("tnb_seq_fuse_cluster", self._standard().handle, self.x_slot.data_ptr(),
                       self.y_slot.data_ptr(), _exec.CLUSTER_CTAS, ctypes.byref(ctas),
                       cl.handle)
             self.cluster, self.cluster_ctas = cl, ctas.value
-        self.fused = None
-        if (not self.uses_tensor_cores and not any(lk.deferred for lk in self.links)
-                and not any(lk.ga is not None for lk in self.links)
-                and 0 < len(std) <= FUSED_MAX_STAGES):
-            from tenet import _lib
-
-            self.barrier = torch.zeros(2, dtype=torch.int32, device=dev)
-            fused = _exec.Seq()
-            _lib.call("tnb_seq_fuse", std.handle, self.x_slot.data_ptr(),
-                      self.y_slot.data_ptr(), self.barrier.data_ptr(), fused.handle)
-            self.fused = fused
         self._built = True
+
+    def _standard(self) -> _exec.Seq:
+        """A chunk-map recording of the chain's stages, the form the one-launch kernels
+        fuse."""
+        if self._std_seq is None:
+            self._std_seq = _exec.Seq()
+            with _exec.standard_gathers(), self._std_seq:
+                self._run_tables(self.x_slot, self.y_slot)
+        return self._std_seq
+
+    @property
+    def fused(self) -> _exec.Seq | None:
+        """The same stages as one persistent launch, built on first use, when they all
+        fuse (no tensor-core stage, no product-source gather, at most the kernel's stage
+        count); else None."""
+        if self._fused is None:
+            self._fused = False
+            if (not self.uses_tensor_cores
+                    and not any(lk.deferred or lk.ga is not None for lk in self.links)
+                    and 0 < len(self.seq) <= FUSED_MAX_STAGES):
+                self.barrier = torch.zeros(2, dtype=torch.int32, device=_exec.device())
+                fused = _exec.Seq()
+                _lib.call("tnb_seq_fuse", self._standard().handle, self.x_slot.data_ptr(),
+                          self.y_slot.data_ptr(), self.barrier.data_ptr(), fused.handle)
+                self._fused = fused
+        return self._fused or None
 
     @property
     def exec_seq(self) -> _exec.Seq:
@@ -389,7 +396,7 @@ class ChainProgram:
         stage-by-stage sequence."""
         if self.cluster is not None and _exec.CLUSTER:
             return self.cluster
-        return self.fused if (self.fused is not None and _exec.FUSE) else self.seq
+        return (self.fused if _exec.FUSE else None) or self.seq
 
     def refresh(self) -> None:
         """Re-pack the fixed operands (after their values changed, same structures)."""
