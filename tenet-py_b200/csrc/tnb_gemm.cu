@@ -24,29 +24,216 @@
 
 namespace tnb {
 
-// K slabs in shared memory per tile shape: 32 x 32 keeps three in flight (33 KB, six CTAs
-// per SM), 64 x 64 two (50 KB, dynamic shared memory).
-template <int TM>
-constexpr int kGemmStages = TM == 64 ? 3 : 4;
+// The tiled kinds run on the FP64 tensor cores: mma.sync m16n8k8 (the tcgen05 unit has no
+// FP64 kind), four warps per tile.  One instruction is 1,024 fused multiply-adds, 64 clocks of
+// its scheduler's FP64 pipe, and a single dependent chain of them per warp already fills the
+// pipe (8.5 of 9.2 TFLOP/s per scheduler over the chip), so four warps saturate an SM and
+// 56 of 64 issue slots stay free for the loads.  The 4 x 4 register tiles of DFMAs that ran
+// here took eight 64-bit shared loads per 16 multiply-adds and topped out at 14-16 TFLOP/s.
+// Each element's products are added in k order in one chain of fused multiply-adds, as
+// before: the same bits (the instruction adds its eight products one after the other).
+//
+// Shared memory: A rows padded to 20 doubles, B rows to TN + 4, so the four k x eight rows (or
+// columns) of a fragment load fall on 32 different banks per half warp.  K slabs of 16 arrive
+// by cp.async, kMmaStages - 1 ahead; all threads read the tile's descriptor row themselves
+// (one broadcast load each, no barrier before the first copy).
+constexpr int kMmaThreads = 128, kMmaStages = 4, kMmaPadA = kBk + 4;
 
 template <int TM, int TN>
-__global__ void __launch_bounds__((TM / 4) * (TN / 4), (TM == 64 ? 1 : 6))
+struct MmaSmem {
+  double As[kMmaStages][TM][kMmaPadA];
+  double Bs[kMmaStages][kBk][TN + 4];
+  int last;
+};
+
+__device__ __forceinline__ void mma_f64(double (&c)[4], const double (&a)[4],
+                                        const double (&b)[2]) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+      "{%0,%1,%2,%3};"
+      : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
+}
+
+// One TM x TN output tile, or one K split of it, by a CTA of four warps in a 2 x 2 grid.
+template <int TM, int TN>
+__global__ void __launch_bounds__(kMmaThreads, (TM == 64 ? 2 : 5))
 gemm_f64_kernel(const GemmArgs g) {
   extern __shared__ __align__(16) uint8_t gemm_smem[];
-  auto& sm = *reinterpret_cast<GemmSmem<TM, TN, kGemmStages<TM>>*>(gemm_smem);
-  gemm_tile<TM, TN, false>(g, blockIdx.x, sm, threadIdx.x, CtaSync{});
+  auto& sm = *reinterpret_cast<MmaSmem<TM, TN>*>(gemm_smem);
+  constexpr int WM = TM / 2, WN = TN / 2;        // a warp's part of the tile
+  constexpr int FM = WM / 16, FN = WN / 8;       // its m16 x n8 fragments
+  constexpr int LA = TM * kBk / kMmaThreads, LB = TN * kBk / kMmaThreads;
+  constexpr int RA = kMmaThreads / kBk, RB = kMmaThreads / TN;  // rows per round of copies
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t tile = blockIdx.x;
+  GemmRow r;
+  bool ok = load_row(g, tile, r);
+  ok = ok && footprint_ok(r, g.n_a, g.n_b, g.n_c);
+  if (ok && r.splits > 1) {
+    const int64_t nt = ((r.M + TM - 1) / TM) * r.tiles_n;
+    ok = r.ksplit > 0 && r.ksplit % kBk == 0 && r.cnt_off >= 0 && r.cnt_off + nt <= g.n_cnt &&
+         r.part_off >= 0 && r.part_off + nt * r.splits * TM * TN <= g.n_parts;
+  }
+  if (!ok) {
+    if (tid == 0) raise_bounds();
+    return;
+  }
+  const int64_t local = tile - r.tile_begin;
+  const int64_t split = local % r.splits, t2 = local / r.splits;
+  const int64_t m0 = (t2 / r.tiles_n) * TM, n0 = (t2 % r.tiles_n) * TN;
+  if (local < 0 || m0 >= r.M || n0 >= r.N) return;
+  const int64_t kb = r.splits > 1 ? split * r.ksplit : 0;
+  const int64_t ke = r.splits > 1 ? min(r.K, kb + r.ksplit) : r.K;
+  const int kn = ke > kb ? static_cast<int>(min(ke - kb, int64_t(INT32_MAX - kBk))) : 0;
+  const int nk = (kn + kBk - 1) / kBk;
+
+  // this thread's copies: A element (ar + RA q, ac), B element (br + RB q, bc) of a slab
+  const int ar = tid / kBk, ac = tid % kBk, br = tid / TN, bc = tid % TN;
+  const double* const pa = g.a + r.aoff + (m0 + ar) * r.lda + kb + ac;
+  const double* const pb = g.b + r.boff + (kb + br) * r.ldb + n0 + bc;
+  const int64_t stepa = RA * r.lda, stepb = RB * r.ldb;
+  const int rows_left = static_cast<int>(min(r.M - m0, int64_t(TM))) - ar;
+  const bool b_in = bc < r.N - n0;
+  auto issue = [&](int s) {
+    const int buf = s % kMmaStages, k0 = s * kBk;
+    const bool a_in = k0 + ac < kn;
+#pragma unroll
+    for (int q = 0; q < LA; ++q) {
+      const bool in = a_in && RA * q < rows_left;
+      cp_async8(&sm.As[buf][ar + RA * q][ac], in ? pa + k0 + q * stepa : g.a, in);
+    }
+#pragma unroll
+    for (int q = 0; q < LB; ++q) {
+      const bool in = b_in && k0 + br + RB * q < kn;
+      cp_async8(&sm.Bs[buf][br + RB * q][bc], in ? pb + k0 * r.ldb + q * stepb : g.b, in);
+    }
+  };
+  double acc[FM][FN][4];
+#pragma unroll
+  for (int i = 0; i < FM; ++i)
+#pragma unroll
+    for (int j = 0; j < FN; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.0;
+
+  pdl_wait();  // A may be the previous kernel's output
+#pragma unroll
+  for (int s = 0; s < kMmaStages - 1; ++s) {
+    if (s < nk) issue(s);
+    cp_async_commit();
+  }
+  const int wm = (warp >> 1) * WM, wn = (warp & 1) * WN, fr = lane >> 2, fk = lane & 3;
+  for (int s = 0; s < nk; ++s) {
+    cp_async_wait<kMmaStages - 2>();  // this thread's copies of slab s have landed
+    __syncthreads();                  // everyone's have, and slab s - 1 is consumed
+    if (s + kMmaStages - 1 < nk) issue(s + kMmaStages - 1);
+    cp_async_commit();
+    const int buf = s % kMmaStages;
+    const int steps = kn - s * kBk > 8 ? 2 : 1;  // (a last slab of up to eight takes one)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (h < steps) {
+        double fa[FM][4], fb[FN][2];
+#pragma unroll
+        for (int i = 0; i < FM; ++i) {
+          const double* p = &sm.As[buf][wm + 16 * i + fr][8 * h + fk];
+          fa[i][0] = p[0];
+          fa[i][1] = p[8 * kMmaPadA];
+          fa[i][2] = p[4];
+          fa[i][3] = p[8 * kMmaPadA + 4];
+        }
+#pragma unroll
+        for (int j = 0; j < FN; ++j) {
+          const double* p = &sm.Bs[buf][8 * h + fk][wn + 8 * j + fr];
+          fb[j][0] = p[0];
+          fb[j][1] = p[4 * (TN + 4)];
+        }
+#pragma unroll
+        for (int i = 0; i < FM; ++i)
+#pragma unroll
+          for (int j = 0; j < FN; ++j) mma_f64(acc[i][j], fa[i], fb[j]);
+      }
+    }
+  }
+  cp_async_wait<0>();
+
+  // element e of fragment (i, j): row 16 i + fr + 8 (e / 2), column 8 j + 2 fk + e % 2
+  if (r.splits > 1) {
+    // split K: park this partial tile, and let the last of the tile's splits to arrive
+    // sum all of them in split order (a fixed order, so the result is deterministic)
+    double* mine = g.parts + r.part_off + (t2 * r.splits + split) * (TM * TN);
+#pragma unroll
+    for (int i = 0; i < FM; ++i)
+#pragma unroll
+      for (int j = 0; j < FN; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          mine[(wm + 16 * i + fr + 8 * (e >> 1)) * TN + wn + 8 * j + 2 * fk + (e & 1)] =
+              acc[i][j][e];
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) {
+      const unsigned int prev = atomicAdd(g.counters + r.cnt_off + t2, 1u);
+      sm.last = (prev == static_cast<unsigned int>(r.splits - 1));
+    }
+    __syncthreads();
+    if (!sm.last) return;
+    __threadfence();
+    const double* base = g.parts + r.part_off + t2 * r.splits * (TM * TN);
+    // splits outermost: each element sums its splits in split order from zero, and one
+    // split's loads are in flight together
+#pragma unroll
+    for (int i = 0; i < FM; ++i)
+#pragma unroll
+      for (int j = 0; j < FN; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.0;
+    for (int64_t q = 0; q < r.splits; ++q) {
+      double v[FM][FN][4];
+#pragma unroll
+      for (int i = 0; i < FM; ++i)
+#pragma unroll
+        for (int j = 0; j < FN; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            v[i][j][e] = __ldcg(base + q * (TM * TN) + (wm + 16 * i + fr + 8 * (e >> 1)) * TN +
+                                wn + 8 * j + 2 * fk + (e & 1));
+#pragma unroll
+      for (int i = 0; i < FM; ++i)
+#pragma unroll
+        for (int j = 0; j < FN; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[i][j][e] += v[i][j][e];
+    }
+    if (tid == 0) g.counters[r.cnt_off + t2] = 0u;  // leave the counters zero for the next run
+  }
+  double* const pc = g.c + r.coff;
+#pragma unroll
+  for (int i = 0; i < FM; ++i)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int64_t gm = m0 + wm + 16 * i + fr + 8 * h;
+      if (gm >= r.M) continue;
+#pragma unroll
+      for (int j = 0; j < FN; ++j) {
+        const int64_t gn = n0 + wn + 8 * j + 2 * fk;
+        if (gn < r.N) pc[gm * r.ldc + gn] = acc[i][j][2 * h];
+        if (gn + 1 < r.N) pc[gm * r.ldc + gn + 1] = acc[i][j][2 * h + 1];
+      }
+    }
 }
 
 template <int TM, int TN>
 cudaError_t launch_gemm_f64(unsigned grid, cudaStream_t s, const GemmArgs& g) {
-  constexpr size_t kSmem = sizeof(GemmSmem<TM, TN, kGemmStages<TM>>);
+  constexpr size_t kSmem = sizeof(MmaSmem<TM, TN>);
   static PerDeviceOnce opted;
   const cudaError_t e = opted.once([] {
     return cudaFuncSetAttribute(gemm_f64_kernel<TM, TN>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
   });
   if (e != cudaSuccess) return e;
-  return launch_dyn(gemm_f64_kernel<TM, TN>, grid, (TM / 4) * (TN / 4), kSmem, s, g);
+  return launch_dyn(gemm_f64_kernel<TM, TN>, grid, kMmaThreads, kSmem, s, g);
 }
 
 __global__ void __launch_bounds__(kSkinnyThreads, 4)
