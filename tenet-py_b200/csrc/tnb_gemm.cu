@@ -6,18 +6,15 @@
 // launch: CTA b reads its (sector, tile) from a tile -> row map, so large and small
 // sectors share the machine in a single wave instead of one launch each.
 //
-// Three tile shapes, chosen by the host per composition:
-//   TNB_TILE_64     64x64 output tile, 256 threads, 4x4 register micro-tile per thread
-//   TNB_TILE_32     32x32 output tile,  64 threads, same micro-tile -- for compositions
-//                   whose 64x64 tiles would not fill the 148 SMs (small M, N, long K)
+// Tile shapes, chosen by the host per composition:
+//   TNB_TILE_64     64x64 output tile, 128 threads
+//   TNB_TILE_32     32x32 output tile, 128 threads -- for compositions whose 64x64 tiles
+//                   would not fill the 148 SMs (small M, N, long K)
 //   TNB_TILE_SKINNY one thread per output row, for products with N <= 16 and K <= 16
 //                   (the MPO links of a matvec: tall, 1-3 columns), B staged in shared
 //                   memory; bandwidth-bound by construction
-//   TNB_TILE_WIDE   one thread per output column, for products with M <= 16 and K <= 16
-//                   (an MPO tensor as the left operand: a few rows, a long N)
-// The plain form computes in FP64 on the DFMA pipe; micro-tile rows/cols are strided so
-// shared-memory reads are conflict-free, and the next K slabs stream into shared memory
-// with cp.async (three ahead for 32 x 32 tiles, two for 64 x 64) while one is consumed.
+//   TNB_TILE_WIDE   a thread per output column (two for K <= 4), for products with M <= 16
+//                   and K <= 16 (an MPO tensor as the left operand: a few rows, a long N)
 #include <string>
 
 #include "tnb_stages.cuh"
@@ -30,6 +27,10 @@ namespace tnb {
 // pipe (8.5 of 9.2 TFLOP/s per scheduler over the chip), so four warps saturate an SM and
 // 56 of 64 issue slots stay free for the loads.  The 4 x 4 register tiles of DFMAs that ran
 // here took eight 64-bit shared loads per 16 multiply-adds and topped out at 14-16 TFLOP/s.
+// Measured on B200: 4096^3 32.3 TFLOP/s (16.4 with DFMA tiles; cuBLAS DGEMM 35.5), a dense
+// U(1) contraction's 1,466 tiles 28.0 (14.4), 3,520 products of about 108 x 82 x 24 8.7 (6.2,
+// then bound by writing C), 95 MFLOP in 335 tiles 8.9 us (17.0).
+//
 // Each element's products are added in k order in one chain of fused multiply-adds, as
 // before: the same bits (the instruction adds its eight products one after the other).
 //
@@ -37,7 +38,7 @@ namespace tnb {
 // columns) of a fragment load fall on 32 different banks per half warp.  K slabs of 16 arrive
 // by cp.async, kMmaStages - 1 ahead; all threads read the tile's descriptor row themselves
 // (one broadcast load each, no barrier before the first copy).
-constexpr int kMmaThreads = 128, kMmaStages = 4, kMmaPadA = kBk + 4;
+constexpr int kMmaThreads = 128, kMmaStages = 3, kMmaPadA = kBk + 4;
 
 template <int TM, int TN>
 struct MmaSmem {
@@ -57,7 +58,7 @@ __device__ __forceinline__ void mma_f64(double (&c)[4], const double (&a)[4],
 
 // One TM x TN output tile, or one K split of it, by a CTA of four warps in a 2 x 2 grid.
 template <int TM, int TN>
-__global__ void __launch_bounds__(kMmaThreads, (TM == 64 ? 2 : 5))
+__global__ void __launch_bounds__(kMmaThreads, (TM == 64 ? 3 : 6))
 gemm_f64_kernel(const GemmArgs g) {
   extern __shared__ __align__(16) uint8_t gemm_smem[];
   auto& sm = *reinterpret_cast<MmaSmem<TM, TN>*>(gemm_smem);
@@ -242,10 +243,63 @@ gemm_f64_skinny_kernel(const GemmArgs g) {
   skinny_tile<kSkinnyThreads, false>(g, blockIdx.x, sm, threadIdx.x, CtaSync{});
 }
 
-__global__ void __launch_bounds__(kSkinnyThreads, 4)
+// kSkinnyThreads output columns, C[:, n] = A * B[:, n] for M, K <= 16 (the transpose of the
+// skinny case: a few rows, a long N), two columns per thread for K <= 4, else one after the
+// other; loads of B and stores of C run along N, so both are coalesced, and A is a handful
+// of broadcast loads.  Bound by HBM: the descriptor row is one round of loads and B's columns
+// the next, with nothing staged between them, and 48 registers keep ten CTAs on an SM.  768
+// products of up to 4 x 25,790 x 4 (474 MB) take 94.6 us, 5.0 TB/s; one column per thread, A
+// staged behind two barriers, took 240 (six CTAs per SM: 131).
+constexpr int kWideThreads = kSkinnyThreads / 2;
+
+template <int KM, int NC>
+__device__ __forceinline__ void wide_columns(const GemmArgs& g, const GemmRow& r, int64_t n) {
+  const int M = static_cast<int>(r.M), K = static_cast<int>(r.K);
+  const double* const pb = g.b + r.boff + n;
+  double bv[NC][KM];
+#pragma unroll
+  for (int c = 0; c < NC; ++c)
+#pragma unroll
+    for (int k = 0; k < KM; ++k)
+      bv[c][k] = k < K && n + c * kWideThreads < r.N ? __ldg(pb + c * kWideThreads + k * r.ldb)
+                                                     : 0.0;
+  const double* const pa = g.a + r.aoff;
+  double* const pc = g.c + r.coff + n;
+#pragma unroll 1
+  for (int m = 0; m < M; ++m) {
+    double s[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) s[c] = 0.0;
+#pragma unroll
+    for (int k = 0; k < KM; ++k)
+      if (k < K) {
+        const double av = __ldg(pa + m * r.lda + k);
+#pragma unroll
+        for (int c = 0; c < NC; ++c) s[c] = fma(av, bv[c][k], s[c]);
+      }
+#pragma unroll
+    for (int c = 0; c < NC; ++c)
+      if (n + c * kWideThreads < r.N) pc[m * r.ldc + c * kWideThreads] = s[c];
+  }
+}
+
+__global__ void __launch_bounds__(kWideThreads, 10)
 gemm_f64_wide_kernel(const GemmArgs g) {
-  __shared__ SkinnySmem sm;
-  wide_tile(g, blockIdx.x, sm);
+  const int64_t tile = blockIdx.x;
+  GemmRow r;
+  if (!load_row(g, tile, r) || !footprint_ok(r, g.n_a, g.n_b, g.n_c) || r.M > kSkinnyMax ||
+      r.K > kSkinnyMax || tile < r.tile_begin) {
+    if (threadIdx.x == 0) raise_bounds();
+    return;
+  }
+  pdl_wait();  // B may be the previous kernel's output
+  const int64_t n = (tile - r.tile_begin) * kSkinnyThreads + threadIdx.x;
+  if (r.K <= 4) {
+    wide_columns<4, 2>(g, r, n);
+  } else {
+#pragma unroll 1
+    for (int c = 0; c < 2; ++c) wide_columns<kSkinnyMax, 1>(g, r, n + c * kWideThreads);
+  }
 }
 
 }  // namespace tnb
@@ -289,7 +343,7 @@ extern "C" int tnb_grouped_gemm_f64(const int64_t* gemm_table, int64_t n_gemm,
       e = tnb::launch(tnb::gemm_f64_skinny_kernel, grid, tnb::kSkinnyThreads, s, g);
       break;
     case TNB_TILE_WIDE:
-      e = tnb::launch(tnb::gemm_f64_wide_kernel, grid, tnb::kSkinnyThreads, s, g);
+      e = tnb::launch(tnb::gemm_f64_wide_kernel, grid, tnb::kWideThreads, s, g);
       break;
     case TNB_TILE_TC_TF32:
     case TNB_TILE_TC_3XBF16:
@@ -343,7 +397,7 @@ extern "C" int tnb_grouped_gemm_f64_rows(const int64_t* tile_rows, int64_t total
       e = tnb::launch(tnb::gemm_f64_skinny_kernel, grid, tnb::kSkinnyThreads, s, g);
       break;
     default:
-      e = tnb::launch(tnb::gemm_f64_wide_kernel, grid, tnb::kSkinnyThreads, s, g);
+      e = tnb::launch(tnb::gemm_f64_wide_kernel, grid, tnb::kWideThreads, s, g);
       break;
   }
   if (e != cudaSuccess) {

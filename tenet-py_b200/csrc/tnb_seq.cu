@@ -132,11 +132,11 @@ __device__ __forceinline__ void run_chain(const FChain& ch, const double* x, dou
                        w[12] > poff ? (w[12] - poff) / 8 : 0};
       if (st.kind == TNB_TILE_64) {
         for (int64_t it = blockIdx.x; it < st.items; it += gridDim.x)
-          gemm_tile<64, 64, true>(g, it, sm.g64, threadIdx.x, CtaSync{});
+          gemm_tile<64, 64>(g, it, sm.g64, threadIdx.x, CtaSync{});
       } else if (st.kind == TNB_TILE_32) {
         for (int64_t it = static_cast<int64_t>(blockIdx.x) * kGroups + grp; it < st.items;
              it += static_cast<int64_t>(gridDim.x) * kGroups)
-          gemm_tile<32, 32, true>(g, it, sm.g32[grp], gtid, gsync);
+          gemm_tile<32, 32>(g, it, sm.g32[grp], gtid, gsync);
       } else {
         for (int64_t it = blockIdx.x; it < st.items; it += gridDim.x)
           skinny_tile<kFusedThreads, true>(g, it, sm.skinny, threadIdx.x, CtaSync{});

@@ -599,15 +599,13 @@ __device__ __forceinline__ bool footprint_ok(const GemmRow& r, int64_t n_a, int6
   return !bad;
 }
 
-// S K slabs of both operands.  The persistent chain kernel uses S = 2 with the next slab
-// prefetched through registers (its sources may have been written earlier in the same
-// launch and are read through L2); a standalone launch keeps S - 1 slabs in flight with
-// cp.async (operands are fixed for the launch), which the DFMA loop needs at the few warps
-// per SM that small coupled sectors give.
-template <int TM, int TN, int S = 2>
+// Two K slabs of both operands, the next one prefetched through registers: the persistent
+// chain kernel's tile, whose sources may have been written earlier in the same launch and
+// are read through L2.  (A standalone launch runs the tensor-core tiles of tnb_gemm.cu.)
+template <int TM, int TN>
 struct GemmSmem {
-  double As[S][kBk][TM + 1];
-  double Bs[S][kBk][TN];
+  double As[2][kBk][TM + 1];
+  double Bs[2][kBk][TN];
   GemmRow row;
   int ok;
   int last;
@@ -628,13 +626,12 @@ __device__ __forceinline__ void cp_async_wait() {
 
 // One TM x TN output tile (or one K split of it) by the NT = TM*TN/16 threads of a group;
 // `tid` is the thread's index within the group.
-template <int TM, int TN, bool kFused, class Sync, int S>
-__device__ void gemm_tile(const GemmArgs& g, int64_t tile, GemmSmem<TM, TN, S>& sm, int tid,
+template <int TM, int TN, class Sync>
+__device__ void gemm_tile(const GemmArgs& g, int64_t tile, GemmSmem<TM, TN>& sm, int tid,
                           Sync sync) {
-  static_assert(!kFused || S == 2, "the persistent kernel double-buffers through registers");
   constexpr int TX = TN / 4, TY = TM / 4, NT = TX * TY;
   constexpr int LA = (TM * kBk) / NT, LB = (TN * kBk) / NT;
-  if constexpr (kFused) sync();  // the previous item's readers are done with sm
+  sync();  // the previous item's readers are done with sm
   if (tid == 0) {
     GemmRow r;
     bool ok = load_row(g, tile, r);
@@ -657,7 +654,6 @@ __device__ void gemm_tile(const GemmArgs& g, int64_t tile, GemmSmem<TM, TN, S>& 
   if (m0 >= r.M || n0 >= r.N) return;
   const int64_t kb = r.splits > 1 ? split * r.ksplit : 0;
   const int64_t ke = r.splits > 1 ? min(r.K, kb + r.ksplit) : r.K;
-  if constexpr (!kFused) pdl_wait();  // A may be the previous kernel's output
 
   const double* __restrict__ a = g.a;
   const double* __restrict__ b = g.b;
@@ -684,7 +680,6 @@ __device__ void gemm_tile(const GemmArgs& g, int64_t tile, GemmSmem<TM, TN, S>& 
   };
   const int64_t nk = ke > kb ? (ke - kb + kBk - 1) / kBk : 0;
 
-  if constexpr (kFused) {
   double ra[LA], rb[LB];
   auto load_slab = [&](int64_t k0) {
 #pragma unroll
@@ -692,14 +687,14 @@ __device__ void gemm_tile(const GemmArgs& g, int64_t tile, GemmSmem<TM, TN, S>& 
       const int idx = tid + q * NT;
       const int am = idx / kBk, ak = idx % kBk;
       const int64_t gm = m0 + am, gk = k0 + ak;
-      ra[q] = (gm < r.M && gk < ke) ? load_data<kFused>(a + r.aoff + gm * r.lda + gk) : 0.0;
+      ra[q] = (gm < r.M && gk < ke) ? load_data<true>(a + r.aoff + gm * r.lda + gk) : 0.0;
     }
 #pragma unroll
     for (int q = 0; q < LB; ++q) {
       const int idx = tid + q * NT;
       const int bk = idx / TN, bn = idx % TN;
       const int64_t gk = k0 + bk, gn = n0 + bn;
-      rb[q] = (gk < ke && gn < r.N) ? load_data<kFused>(b + r.boff + gk * r.ldb + gn) : 0.0;
+      rb[q] = (gk < ke && gn < r.N) ? load_data<true>(b + r.boff + gk * r.ldb + gn) : 0.0;
     }
   };
   auto store_slab = [&](int buf) {
@@ -726,44 +721,6 @@ __device__ void gemm_tile(const GemmArgs& g, int64_t tile, GemmSmem<TM, TN, S>& 
     slab_fma(cur);
     if (s + 1 < nk) store_slab(cur ^ 1);
     sync();
-  }
-  } else {
-  // slab s lands in buffer s % S; S - 1 slabs are in flight while one is consumed
-  const double* const a0 = a + r.aoff;
-  const double* const b0 = b + r.boff;
-  auto issue = [&](int64_t s) {
-    const int buf = static_cast<int>(s % S);
-    const int64_t k0 = kb + s * kBk;
-#pragma unroll
-    for (int q = 0; q < LA; ++q) {
-      const int idx = tid + q * NT;
-      const int am = idx / kBk, ak = idx % kBk;
-      const int64_t gm = m0 + am, gk = k0 + ak;
-      const bool ok = gm < r.M && gk < ke;
-      cp_async8(&sm.As[buf][ak][am], ok ? a0 + gm * r.lda + gk : a0, ok);
-    }
-#pragma unroll
-    for (int q = 0; q < LB; ++q) {
-      const int idx = tid + q * NT;
-      const int bk = idx / TN, bn = idx % TN;
-      const int64_t gk = k0 + bk, gn = n0 + bn;
-      const bool ok = gk < ke && gn < r.N;
-      cp_async8(&sm.Bs[buf][bk][bn], ok ? b0 + gk * r.ldb + gn : b0, ok);
-    }
-  };
-#pragma unroll
-  for (int s = 0; s < S - 1; ++s) {
-    if (s < nk) issue(s);
-    cp_async_commit();
-  }
-  for (int64_t s = 0; s < nk; ++s) {
-    cp_async_wait<S - 2>();  // this thread's copies of slab s have landed
-    sync();                  // everyone's have, and slab s - 1 is consumed
-    if (s + S - 1 < nk) issue(s + S - 1);
-    cp_async_commit();
-    slab_fma(static_cast<int>(s % S));
-  }
-  cp_async_wait<0>();
   }
 
   if (r.splits > 1) {
@@ -872,42 +829,6 @@ __device__ void skinny_tile(const GemmArgs& g, int64_t tile, SkinnySmem& sm, int
         g.c[r.coff + m * r.ldc + n] = s;
       }
     }
-  }
-}
-
-// kSkinnyThreads output columns, C[:, n] = A * B[:, n] for M, K <= 16, one column per
-// thread (the transpose of the skinny case: a few rows, a long N): A is staged in shared
-// memory, and loads of B and stores of C run along N, so both are coalesced.
-__device__ inline void wide_tile(const GemmArgs& g, int64_t tile, SkinnySmem& sm) {
-  const int tid = threadIdx.x;
-  if (tid == 0) {
-    GemmRow r;
-    bool ok = load_row(g, tile, r);
-    ok = ok && footprint_ok(r, g.n_a, g.n_b, g.n_c) && r.M <= kSkinnyMax && r.K <= kSkinnyMax;
-    if (!ok) raise_bounds();
-    sm.row = r;
-    sm.ok = ok;
-  }
-  __syncthreads();
-  if (!sm.ok) return;
-  const GemmRow r = sm.row;
-  const int M = static_cast<int>(r.M), K = static_cast<int>(r.K);
-  pdl_wait();  // B may be the previous kernel's output
-  for (int i = tid; i < M * K; i += kSkinnyThreads)
-    sm.Bs[i] = __ldg(g.a + r.aoff + (i / K) * r.lda + (i % K));
-  __syncthreads();
-  const int64_t n = (tile - r.tile_begin) * kSkinnyThreads + tid;
-  if (n >= r.N) return;
-  double bv[kSkinnyMax];
-#pragma unroll
-  for (int k = 0; k < kSkinnyMax; ++k) bv[k] = k < K ? __ldg(g.b + r.boff + k * r.ldb + n) : 0.0;
-#pragma unroll 1
-  for (int m = 0; m < M; ++m) {
-    double s = 0.0;
-#pragma unroll
-    for (int k = 0; k < kSkinnyMax; ++k)
-      if (k < K) s = fma(sm.Bs[m * K + k], bv[k], s);
-    g.c[r.coff + m * r.ldc + n] = s;
   }
 }
 
