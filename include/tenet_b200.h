@@ -228,6 +228,18 @@ int tnb_grouped_gemm_f64_rows(const int64_t* tile_rows, int64_t total_tiles, int
                               int64_t n_counters, void* stream);
 
 /*
+ * The tensor-core kinds with each packed slab described by a row of four int64: the slab's
+ * first element in its operand, the operand's leading dimension, rows | K columns << 32, 0
+ * (A slabs, then B slabs, in the order of their chunks): the pack kernel then searches no
+ * table.  Everything else as tnb_grouped_gemm_f64.
+ */
+int tnb_grouped_gemm_tc(const int64_t* gemm_table, int64_t n_gemm, const int32_t* tile_map,
+                        int64_t total_tiles, const int64_t* slab_rows, int32_t tile_kind,
+                        const double* a, int64_t n_a, const double* b, int64_t n_b, double* c,
+                        int64_t n_c, void* work, int64_t work_bytes, int64_t n_counters,
+                        void* stream);
+
+/*
  * A grouped FP64 GEMM whose A operand is a gather evaluated where it is read: the
  * to_matrices / repartition of the left operand (map_view.py:238-279,
  * ops/repartition.py:458-476) and compose's per-sector matmul (ops/map.py:155-172) in

@@ -347,8 +347,8 @@ extern "C" int tnb_grouped_gemm_f64(const int64_t* gemm_table, int64_t n_gemm,
       break;
     case TNB_TILE_TC_TF32:
     case TNB_TILE_TC_3XBF16:
-      e = tnb::launch_gemm_tc(tile_kind, grid, s, gemm_table, n_gemm, tile_map, a, n_a, b, n_b,
-                              c, n_c, work, work_bytes, n_counters);
+      e = tnb::launch_gemm_tc(tile_kind, grid, s, gemm_table, n_gemm, tile_map, nullptr, a, n_a,
+                              b, n_b, c, n_c, work, work_bytes, n_counters);
       break;
     default:
       tnb::set_error("tnb_grouped_gemm_f64: unknown tile kind");
@@ -405,4 +405,31 @@ extern "C" int tnb_grouped_gemm_f64_rows(const int64_t* tile_rows, int64_t total
     return TNB_ECUDA;
   }
   return tnb::check_launch("tnb_grouped_gemm_f64_rows");
+}
+
+extern "C" int tnb_grouped_gemm_tc(const int64_t* gemm_table, int64_t n_gemm,
+                                   const int32_t* tile_map, int64_t total_tiles,
+                                   const int64_t* slab_rows, int32_t tile_kind, const double* a,
+                                   int64_t n_a, const double* b, int64_t n_b, double* c,
+                                   int64_t n_c, void* work, int64_t work_bytes,
+                                   int64_t n_counters, void* stream) {
+  TNB_REQUIRE(n_gemm >= 0 && total_tiles >= 0, "tnb_grouped_gemm_tc: negative size");
+  if (n_gemm == 0 || total_tiles == 0) return TNB_OK;
+  TNB_REQUIRE(gemm_table != nullptr && tile_map != nullptr && c != nullptr,
+              "tnb_grouped_gemm_tc: null table, tile map or C");
+  TNB_REQUIRE(total_tiles < (int64_t(1) << 31), "tnb_grouped_gemm_tc: too many tiles");
+  TNB_REQUIRE(tile_kind == TNB_TILE_TC_TF32 || tile_kind == TNB_TILE_TC_3XBF16,
+              "tnb_grouped_gemm_tc: tensor-core tile kinds only");
+  const int64_t n_slabs = (n_counters & 0xFFFFFFFFll) + (n_counters >> 32);
+  TNB_REQUIRE(work_bytes >= 0 && n_counters >= 0 && (work_bytes == 0 || work != nullptr) &&
+                  n_slabs * 16384 <= work_bytes && (n_slabs == 0 || slab_rows != nullptr),
+              "tnb_grouped_gemm_tc: bad work buffer or slab rows");
+  const cudaError_t e = tnb::launch_gemm_tc(
+      tile_kind, static_cast<unsigned>(total_tiles), tnb::as_stream(stream), gemm_table, n_gemm,
+      tile_map, slab_rows, a, n_a, b, n_b, c, n_c, work, work_bytes, n_counters);
+  if (e != cudaSuccess) {
+    tnb::set_error(std::string("tnb_grouped_gemm_tc: ") + cudaGetErrorString(e));
+    return TNB_ECUDA;
+  }
+  return tnb::check_launch("tnb_grouped_gemm_tc");
 }

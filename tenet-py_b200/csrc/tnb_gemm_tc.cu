@@ -13,7 +13,10 @@
 // 32 slab of A (and of B^T) becomes one 16 KB chunk of the work buffer, already in the
 // canonical K-major, no-swizzle UMMA shared-memory layout (8-row x 16-byte core
 // matrices, LBO = 128 B between the two core matrices of one K step, SBO between 8-row
-// groups), parts (BF16 hi, lo) back to back.  The MMA kernel gives each CTA a 128 x 128
+// groups), parts (BF16 hi, lo) back to back.  Only the 8-row groups that hold rows of the
+// operand are written and later copied (a prefix of each part): a row past M or N only
+// reaches accumulators that are never stored, and the sectors of a symmetric tensor fill
+// 14 to 40 of 128 rows.  The MMA kernel gives each CTA a 128 x 128
 // output tile and runs a three-stage pipeline: one producer thread copies the next A and
 // B slabs with cp.async.bulk (global -> shared, completion counted in bytes on the
 // stage's "full" mbarrier), one issuer thread waits for "full", issues the MMAs into a
@@ -100,93 +103,126 @@ __device__ __forceinline__ bool load_t2row(const int64_t* table, int64_t g, T2Ro
   return r.M >= 0 && r.N >= 0 && r.K >= 0 && r.a_chunk >= 0 && r.b_chunk >= 0;
 }
 
-// The table row owning packed chunk `chunk` of operand A (which == 0) or B (which == 1):
-// the last row whose first chunk is <= chunk (rows in chunk order).
-__device__ int64_t owner_row(const int64_t* table, int64_t n_gemm, int64_t chunk, int which) {
-  int64_t lo = 0, hi = n_gemm - 1;
-  while (lo < hi) {
-    const int64_t mid = (lo + hi + 1) >> 1;
-    if (table[mid * TNB_GEMM_WIDTH + 12 + which] <= chunk) lo = mid; else hi = mid - 1;
+// One packed slab: its first element in the operand, the operand's leading dimension, and how
+// many of its 128 rows and 32 columns of K the operand has.
+struct Slab {
+  int64_t off, ld;
+  int rows, cols;
+};
+
+// The slab `chunk` of operand A (which == 0) or B (which == 1) from the GEMM table: its row
+// is the last one whose first chunk is <= chunk (rows in chunk order), found by the warp in
+// ceil(log32 n_gemm) rounds of 32 probes.
+__device__ Slab find_slab(const int64_t* table, int64_t n_gemm, int64_t chunk, int which,
+                          int lane) {
+  int64_t lo = 0, n = n_gemm;  // the row is in [lo, lo + n)
+  while (n > 1) {
+    const int64_t step = (n + 31) / 32;
+    const bool before = lane * step < n &&
+                        table[(lo + lane * step) * TNB_GEMM_WIDTH + 12 + which] <= chunk;
+    const int last = 31 - __clz(__ballot_sync(0xffffffffu, before || lane == 0));
+    n = min(step, n - last * step);
+    lo += last * step;
   }
-  return lo;
+  T2Row r;
+  Slab s{0, 0, 0, 0};
+  if (!load_t2row(table, lo, r)) return s;
+  const int64_t ks = (r.K + kT2Bk - 1) / kT2Bk;
+  const int64_t local = chunk - (which == 0 ? r.a_chunk : r.b_chunk);
+  const int64_t rows = which == 0 ? r.M : r.N;
+  if (ks == 0 || local < 0) return s;
+  const int64_t t0 = (local / ks) * kT2M, k0 = (local % ks) * kT2Bk;
+  if (t0 >= rows) return s;
+  s.ld = which == 0 ? r.lda : r.ldb;
+  s.off = which == 0 ? r.aoff + t0 * s.ld + k0 : r.boff + k0 * s.ld + t0;
+  s.rows = static_cast<int>(min(rows - t0, int64_t(kT2M)));
+  s.cols = static_cast<int>(min(r.K - k0, int64_t(kT2Bk)));
+  return s;
 }
 
-// Pack one 128 x 32 slab of A (blocks [0, a_chunks): rows = M, read along K) or of B^T
-// (blocks after them: rows = N, read along N) into its work-buffer chunk in the UMMA
-// layout.  Each of the 256 threads loads its 16 elements at once (coalesced along the
-// operand's contiguous dimension), the slab is assembled in shared memory and leaves as
-// 16-byte stores.
-constexpr int kPackThreads = 256, kPackPer = (kT2M * kT2Bk) / kPackThreads;
+// Eight consecutive K elements of one slab row in the UMMA layout: one 16-byte store per
+// BF16 part, or two of TF32.
+template <int MODE>
+__device__ __forceinline__ void pack_eight(uint8_t* slab, int row, int kg, const double (&x)[8]) {
+  using L = T2Layout<MODE>;
+  if constexpr (MODE == 0) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      uint4 v;
+      v.x = to_tf32(x[4 * h]);
+      v.y = to_tf32(x[4 * h + 1]);
+      v.z = to_tf32(x[4 * h + 2]);
+      v.w = to_tf32(x[4 * h + 3]);
+      *reinterpret_cast<uint4*>(slab + kmajor(row, 8 * kg + 4 * h, L::kEsz, L::kRowBytes)) = v;
+    }
+  } else {
+    __align__(16) __nv_bfloat16 hi[8], lo[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      hi[j] = __double2bfloat16(x[j]);
+      lo[j] = __double2bfloat16(x[j] - static_cast<double>(__bfloat162float(hi[j])));
+    }
+    uint8_t* const p = slab + kmajor(row, 8 * kg, L::kEsz, L::kRowBytes);
+    *reinterpret_cast<uint4*>(p) = *reinterpret_cast<const uint4*>(hi);
+    *reinterpret_cast<uint4*>(p + L::kPartBytes) = *reinterpret_cast<const uint4*>(lo);
+  }
+}
+
+// Pack one slab of A (blocks [0, a_chunks): rows = M, read along K) or of B^T (blocks after
+// them: rows = N, read along N) into its work-buffer chunk.  Warps work alone: one takes 8
+// rows x 32 K of A or 32 rows x 8 K of B at a time, a lane eight K elements of one row, all
+// eight loads in flight, and stores whole 16-byte core-matrix rows (a warp's stores fill 512
+// contiguous bytes of A, 128-byte runs of B).  `slabs` (four words per slab: Slab with rows |
+// cols << 32) makes a slab's description one load; without it each warp searches the table.
+// Measured (before: slabs assembled element by element in shared memory behind a 12-step
+// binary search, whole slabs written): the operands of the 64-member environment update's two
+// products 130 us in all (566; 462 with the 32-way search alone), of a dense U(1) contraction
+// 21 us (35).
+constexpr int kPackThreads = 256;
 
 template <int MODE>
 __global__ void __launch_bounds__(kPackThreads)
-tc_pack_kernel(const int64_t* __restrict__ table, int64_t n_gemm, const double* __restrict__ a,
-               int64_t n_a, const double* __restrict__ b, int64_t n_b,
-               uint8_t* __restrict__ work, int64_t work_bytes, int64_t a_chunks) {
-  using L = T2Layout<MODE>;
-  __shared__ __align__(16) uint8_t slab[kT2Slab];
-  __shared__ T2Row s_row;
-  __shared__ int s_ok;
-  const int tid = threadIdx.x;
+tc_pack_kernel(const int64_t* __restrict__ table, int64_t n_gemm,
+               const int64_t* __restrict__ slabs, const double* __restrict__ a, int64_t n_a,
+               const double* __restrict__ b, int64_t n_b, uint8_t* __restrict__ work,
+               int64_t work_bytes, int64_t a_chunks) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int which = blockIdx.x < a_chunks ? 0 : 1;
-  const int64_t chunk = which == 0 ? blockIdx.x : blockIdx.x - a_chunks;
-  if (tid == 0) {
-    T2Row r{};
-    const int64_t g = owner_row(table, n_gemm, chunk, which);
-    bool ok = load_t2row(table, g, r);
-    const int64_t rows = which == 0 ? r.M : r.N;
-    const int64_t ks = (r.K + kT2Bk - 1) / kT2Bk;
-    ok = ok && ks > 0 && (static_cast<int64_t>(blockIdx.x) + 1) * kT2Slab <= work_bytes;
-    if (ok) {  // the row's operand footprint
-      ok = which == 0 ? (r.aoff >= 0 && r.aoff + (r.M - 1) * r.lda + r.K <= n_a)
-                      : (r.boff >= 0 && r.boff + (r.K - 1) * r.ldb + r.N <= n_b);
-      ok = ok && rows > 0;
-    }
-    if (!ok) raise_bounds();
-    s_row = r;
-    s_ok = ok;
+  Slab s;
+  if (slabs != nullptr) {
+    const int64_t* w = slabs + static_cast<int64_t>(blockIdx.x) * 4;
+    s.off = __ldg(w);
+    s.ld = __ldg(w + 1);
+    const int64_t rc = __ldg(w + 2);
+    s.rows = static_cast<int>(rc);
+    s.cols = static_cast<int>(rc >> 32);
+  } else {
+    s = find_slab(table, n_gemm, which == 0 ? blockIdx.x : blockIdx.x - a_chunks, which, lane);
   }
-  __syncthreads();
-  if (!s_ok) return;
-  const T2Row r = s_row;
-  const int64_t ks = (r.K + kT2Bk - 1) / kT2Bk;
-  const int64_t local = chunk - (which == 0 ? r.a_chunk : r.b_chunk);
-  const int64_t t0 = (local / ks) * kT2M, k0 = (local % ks) * kT2Bk;
+  // the slab's own rows and columns inside the operand, its chunk inside the work buffer
+  const int64_t last = which == 0 ? s.off + (s.rows - 1) * s.ld + s.cols
+                                  : s.off + (s.cols - 1) * s.ld + s.rows;
+  if (s.rows < 1 || s.rows > kT2M || s.cols < 1 || s.cols > kT2Bk || s.off < 0 || s.ld < 0 ||
+      last > (which == 0 ? n_a : n_b) ||
+      (static_cast<int64_t>(blockIdx.x) + 1) * kT2Slab > work_bytes) {
+    if (threadIdx.x == 0) raise_bounds();
+    return;
+  }
+  uint8_t* const slab = work + static_cast<int64_t>(blockIdx.x) * kT2Slab;
   pdl_wait();  // the operand may be the previous kernel's output
-  double x[kPackPer];
+  const double* const src = (which == 0 ? a : b) + s.off;
+  const int pieces = which == 0 ? (s.rows + 7) / 8 : 4 * ((s.rows + 31) / 32);
+  for (int i = warp; i < pieces; i += kPackThreads / 32) {
+    const int row = which == 0 ? 8 * i + (lane & 7) : 32 * (i >> 2) + lane;
+    const int kg = which == 0 ? lane >> 3 : i & 3;
+    const int64_t at = which == 0 ? row * s.ld + 8 * kg : 8 * kg * s.ld + row;
+    const int64_t step = which == 0 ? 1 : s.ld;
+    double x[8];
 #pragma unroll
-  for (int i = 0; i < kPackPer; ++i) {
-    const int idx = tid + i * kPackThreads;
-    if (which == 0) {  // A: consecutive threads along K
-      const int64_t gm = t0 + idx / kT2Bk, gk = k0 + idx % kT2Bk;
-      x[i] = (gm < r.M && gk < r.K) ? __ldg(a + r.aoff + gm * r.lda + gk) : 0.0;
-    } else {  // B: consecutive threads along N
-      const int64_t gk = k0 + idx / kT2N, gn = t0 + idx % kT2N;
-      x[i] = (gk < r.K && gn < r.N) ? __ldg(b + r.boff + gk * r.ldb + gn) : 0.0;
-    }
+    for (int j = 0; j < 8; ++j)
+      x[j] = row < s.rows && 8 * kg + j < s.cols ? __ldg(src + at + j * step) : 0.0;
+    if (row < ((s.rows + 7) & ~7)) pack_eight<MODE>(slab, row, kg, x);
   }
-#pragma unroll
-  for (int i = 0; i < kPackPer; ++i) {
-    const int idx = tid + i * kPackThreads;
-    const int rr = which == 0 ? idx / kT2Bk : idx % kT2N;
-    const int kk = which == 0 ? idx % kT2Bk : idx / kT2N;
-    const uint32_t off = kmajor(rr, kk, L::kEsz, L::kRowBytes);
-    if constexpr (MODE == 0) {
-      *reinterpret_cast<uint32_t*>(slab + off) = to_tf32(x[i]);
-    } else {
-      const __nv_bfloat16 hi = __double2bfloat16(x[i]);
-      const __nv_bfloat16 lo =
-          __double2bfloat16(x[i] - static_cast<double>(__bfloat162float(hi)));
-      *reinterpret_cast<__nv_bfloat16*>(slab + off) = hi;
-      *reinterpret_cast<__nv_bfloat16*>(slab + L::kPartBytes + off) = lo;
-    }
-  }
-  __syncthreads();
-  uint4* dst = reinterpret_cast<uint4*>(work + static_cast<int64_t>(blockIdx.x) * kT2Slab);
-  const uint4* from = reinterpret_cast<const uint4*>(slab);
-#pragma unroll
-  for (int i = 0; i < kT2Slab / 16 / kPackThreads; ++i)
-    dst[tid + i * kPackThreads] = from[tid + i * kPackThreads];
 }
 
 __device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes,
@@ -252,6 +288,11 @@ tc_mma_kernel(const int64_t* __restrict__ table, int64_t n_gemm,
   const int64_t nk = ok ? (r.K + kT2Bk - 1) / kT2Bk : 0;
   const uint8_t* a_src = work + (r.a_chunk + mtile * nk) * kT2Slab;
   const uint8_t* b_src = work + (b_chunk0 + r.b_chunk + ntile * nk) * kT2Slab;
+  // bytes of a part's written 8-row groups (nothing past them is read into a stored element)
+  const int rows_a = ok ? static_cast<int>(min(r.M - mtile * kT2M, int64_t(kT2M))) : 0;
+  const int rows_b = ok ? static_cast<int>(min(r.N - ntile * kT2N, int64_t(kT2N))) : 0;
+  const uint32_t bytes_a = static_cast<uint32_t>(((rows_a + 7) & ~7) * L::kRowBytes);
+  const uint32_t bytes_b = static_cast<uint32_t>(((rows_b + 7) & ~7) * L::kRowBytes);
   pdl_wait();  // the packed operands are the pack kernels' output
 
   if (tid == 0 && nk > 0) {  // producer
@@ -268,10 +309,14 @@ tc_mma_kernel(const int64_t* __restrict__ table, int64_t n_gemm,
       }
       const uint32_t fb = smem_u32(&full[st]);
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
-                   :: "r"(fb), "r"(static_cast<uint32_t>(2 * kT2Slab)) : "memory");
+                   :: "r"(fb), "r"(L::kParts * (bytes_a + bytes_b)) : "memory");
       const uint32_t sa = smem_u32(smem + st * L::kStageBytes);
-      bulk_copy(sa, a_src + s * kT2Slab, kT2Slab, fb);
-      bulk_copy(sa + kT2Slab, b_src + s * kT2Slab, kT2Slab, fb);
+#pragma unroll
+      for (int p = 0; p < L::kParts; ++p) {
+        bulk_copy(sa + p * L::kPartBytes, a_src + s * kT2Slab + p * L::kPartBytes, bytes_a, fb);
+        bulk_copy(sa + kT2Slab + p * L::kPartBytes, b_src + s * kT2Slab + p * L::kPartBytes,
+                  bytes_b, fb);
+      }
       s_fills = static_cast<int>(s + 1);
     }
   } else if (tid == 32 && nk > 0) {  // MMA issuer
@@ -395,7 +440,7 @@ tc_mma_kernel(const int64_t* __restrict__ table, int64_t n_gemm,
 
 template <int MODE>
 cudaError_t launch_tc_mode(unsigned grid, cudaStream_t s, const int64_t* table, int64_t n_gemm,
-                           const int32_t* tile_map, const double* a, int64_t n_a,
+                           const int32_t* tile_map, const int64_t* slabs, const double* a, int64_t n_a,
                            const double* b, int64_t n_b, double* c, int64_t n_c, void* work,
                            int64_t work_bytes, int64_t a_chunks, int64_t b_chunks) {
   using L = T2Layout<MODE>;
@@ -408,7 +453,7 @@ cudaError_t launch_tc_mode(unsigned grid, cudaStream_t s, const int64_t* table, 
   auto* w = static_cast<uint8_t*>(work);
   if (a_chunks + b_chunks > 0)
     e = launch(tc_pack_kernel<MODE>, static_cast<unsigned>(a_chunks + b_chunks), kPackThreads, s,
-               table, n_gemm, a, n_a, b, n_b, w, work_bytes, a_chunks);
+               table, n_gemm, slabs, a, n_a, b, n_b, w, work_bytes, a_chunks);
   if (e == cudaSuccess)
     e = launch_dyn(tc_mma_kernel<MODE>, grid, kT2Threads, L::kSmemBytes, s, table, n_gemm,
                    tile_map, static_cast<const uint8_t*>(w), work_bytes, a_chunks, c, n_c);
@@ -416,16 +461,16 @@ cudaError_t launch_tc_mode(unsigned grid, cudaStream_t s, const int64_t* table, 
 }
 
 cudaError_t launch_gemm_tc(int kind, unsigned grid, cudaStream_t s, const int64_t* table,
-                           int64_t n_gemm, const int32_t* tile_map, const double* a,
-                           int64_t n_a, const double* b, int64_t n_b, double* c, int64_t n_c,
+                           int64_t n_gemm, const int32_t* tile_map, const int64_t* slabs,
+                           const double* a, int64_t n_a, const double* b, int64_t n_b, double* c, int64_t n_c,
                            void* work, int64_t work_bytes, int64_t n_counters) {
   const int64_t a_chunks = n_counters & 0xFFFFFFFFll, b_chunks = (n_counters >> 32) & 0xFFFFFFFFll;
   if ((a_chunks + b_chunks) * kT2Slab > work_bytes || ((a_chunks + b_chunks) > 0 && !work))
     return cudaErrorInvalidValue;
   if (kind == TNB_TILE_TC_TF32)
-    return launch_tc_mode<0>(grid, s, table, n_gemm, tile_map, a, n_a, b, n_b, c, n_c, work,
+    return launch_tc_mode<0>(grid, s, table, n_gemm, tile_map, slabs, a, n_a, b, n_b, c, n_c, work,
                              work_bytes, a_chunks, b_chunks);
-  return launch_tc_mode<1>(grid, s, table, n_gemm, tile_map, a, n_a, b, n_b, c, n_c, work,
+  return launch_tc_mode<1>(grid, s, table, n_gemm, tile_map, slabs, a, n_a, b, n_b, c, n_c, work,
                            work_bytes, a_chunks, b_chunks);
 }
 

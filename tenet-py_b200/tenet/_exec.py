@@ -811,6 +811,25 @@ class GemmTable:
             self._dev = Uploaded(self.host_arrays())
         return self._dev.ready()
 
+    def slab_rows(self) -> np.ndarray:
+        """The packed slabs of a tensor-core table (``tnb_grouped_gemm_tc``): per slab its
+        first element, leading dimension and ``rows | K columns << 32``, A's slabs first."""
+        out = []
+        t = self.table
+        ks = (t[:, 2] + TC_BK - 1) // TC_BK
+        for rows, off, ld, along in ((t[:, 0], t[:, 3], t[:, 4], 0), (t[:, 1], t[:, 5], t[:, 6], 1)):
+            tiles = (rows + TC_TILE - 1) // TC_TILE
+            own = np.repeat(np.arange(len(t)), tiles * ks)
+            local = np.arange(len(own)) - np.repeat(np.cumsum(tiles * ks) - tiles * ks, tiles * ks)
+            t0, k0 = local // np.maximum(ks[own], 1) * TC_TILE, local % np.maximum(ks[own], 1) * TC_BK
+            s = np.zeros((len(own), 4), np.int64)
+            s[:, 0] = off[own] + (t0 * ld[own] + k0 if along == 0 else k0 * ld[own] + t0)
+            s[:, 1] = ld[own]
+            s[:, 2] = (np.minimum(rows[own] - t0, TC_TILE)
+                       | np.minimum(t[own, 2] - k0, TC_BK) << 32)
+            out.append(s)
+        return np.concatenate(out)
+
     def tile_rows(self) -> np.ndarray:
         """The table as one row per tile (``tnb_grouped_gemm_f64_rows``)."""
         return np.ascontiguousarray(self.table[self.tile_map])
@@ -833,6 +852,18 @@ class GemmTable:
                       self.work_bytes, self.n_counters, stream_ptr())
             if _LOG is not None:
                 _LOG.end("grouped_gemm_f64", mark, self.flops)
+            return
+        if rec is None and self.kind in (TILE_TC_TF32, TILE_TC_3XBF16) and self.n_counters \
+                and self.tiles >= DIRECT_MIN_TILES:
+            if self._rows_dev is None:
+                self._rows_dev = Uploaded((self.table, self.tile_map, self.slab_rows()))
+            table, tile_map, slabs = self._rows_dev.ready()
+            mark = _LOG.begin() if _LOG is not None else None
+            _lib.call("tnb_grouped_gemm_tc", ptr(table), self.n_gemm, ptr(tile_map), self.tiles,
+                      ptr(slabs), self.kind, ptr(a), a.numel(), ptr(b), b.numel(), ptr(c),
+                      c.numel(), ptr(work), self.work_bytes, self.n_counters, stream_ptr())
+            if _LOG is not None:
+                _LOG.end("grouped_gemm_tc", mark, self.flops)
             return
         table, tile_map = self.device_tables()
         if rec is not None:

@@ -76,3 +76,16 @@ def test_wide(K):
     rng = np.random.default_rng(K)
     shapes = [(m, n, K) for m in (1, 4, 16) for n in (1, 127, 128, 129, 255, 256, 257, 600)]
     _check(*_products(rng, shapes), _exec.TILE_WIDE, False)
+
+
+@pytest.mark.parametrize("precision", ["tf32", "3xbf16"])
+@pytest.mark.parametrize("rows", [1, 2, 31, 32, 33, 1025])
+def test_packed_slabs_of_many_rows(precision, rows):
+    """Tensor-core tables of every size class of the pack kernel's search for a slab's row:
+    integers of up to 3 bits are exact in either form."""
+    rng = np.random.default_rng(rows)
+    shapes = [(int(m), int(n), int(k)) for m, n, k in
+              zip(rng.integers(1, 140, rows), rng.integers(1, 140, rows),
+                  rng.choice([0, 1, 31, 32, 33, 70], rows))]
+    prods, a, b, want, n_c = _products(rng, shapes)
+    _check(prods, a, b, want, n_c, _exec.TC_KINDS[precision], False)
