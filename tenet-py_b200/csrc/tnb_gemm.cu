@@ -56,110 +56,17 @@ __device__ __forceinline__ void mma_f64(double (&c)[4], const double (&a)[4],
       : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
 }
 
-// One TM x TN output tile, or one K split of it, by a CTA of four warps in a 2 x 2 grid.
+// The fragments of a finished tile (or K split of one) into C.  Element e of fragment (i, j) of
+// a warp: row 16 i + lane / 4 + 8 (e / 2), column 8 j + 2 (lane % 4) + e % 2 of its part.
 template <int TM, int TN>
-__global__ void __launch_bounds__(kMmaThreads, (TM == 64 ? 3 : 6))
-gemm_f64_kernel(const GemmArgs g) {
-  extern __shared__ __align__(16) uint8_t gemm_smem[];
-  auto& sm = *reinterpret_cast<MmaSmem<TM, TN>*>(gemm_smem);
-  constexpr int WM = TM / 2, WN = TN / 2;        // a warp's part of the tile
-  constexpr int FM = WM / 16, FN = WN / 8;       // its m16 x n8 fragments
-  constexpr int LA = TM * kBk / kMmaThreads, LB = TN * kBk / kMmaThreads;
-  constexpr int RA = kMmaThreads / kBk, RB = kMmaThreads / TN;  // rows per round of copies
+__device__ __forceinline__ void flush_tile(const GemmArgs& g, const GemmRow& r, int64_t t2,
+                                           int64_t split, int64_t m0, int64_t n0,
+                                           double (&acc)[TM / 32][TN / 16][4],
+                                           MmaSmem<TM, TN>& sm) {
+  constexpr int FM = TM / 32, FN = TN / 16;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t tile = blockIdx.x;
-  GemmRow r;
-  bool ok = load_row(g, tile, r);
-  ok = ok && footprint_ok(r, g.n_a, g.n_b, g.n_c);
-  if (ok && r.splits > 1) {
-    const int64_t nt = ((r.M + TM - 1) / TM) * r.tiles_n;
-    ok = r.ksplit > 0 && r.ksplit % kBk == 0 && r.cnt_off >= 0 && r.cnt_off + nt <= g.n_cnt &&
-         r.part_off >= 0 && r.part_off + nt * r.splits * TM * TN <= g.n_parts;
-  }
-  if (!ok) {
-    if (tid == 0) raise_bounds();
-    return;
-  }
-  const int64_t local = tile - r.tile_begin;
-  const int64_t split = local % r.splits, t2 = local / r.splits;
-  const int64_t m0 = (t2 / r.tiles_n) * TM, n0 = (t2 % r.tiles_n) * TN;
-  if (local < 0 || m0 >= r.M || n0 >= r.N) return;
-  const int64_t kb = r.splits > 1 ? split * r.ksplit : 0;
-  const int64_t ke = r.splits > 1 ? min(r.K, kb + r.ksplit) : r.K;
-  const int kn = ke > kb ? static_cast<int>(min(ke - kb, int64_t(INT32_MAX - kBk))) : 0;
-  const int nk = (kn + kBk - 1) / kBk;
-
-  // this thread's copies: A element (ar + RA q, ac), B element (br + RB q, bc) of a slab
-  const int ar = tid / kBk, ac = tid % kBk, br = tid / TN, bc = tid % TN;
-  const double* const pa = g.a + r.aoff + (m0 + ar) * r.lda + kb + ac;
-  const double* const pb = g.b + r.boff + (kb + br) * r.ldb + n0 + bc;
-  const int64_t stepa = RA * r.lda, stepb = RB * r.ldb;
-  const int rows_left = static_cast<int>(min(r.M - m0, int64_t(TM))) - ar;
-  const bool b_in = bc < r.N - n0;
-  auto issue = [&](int s) {
-    const int buf = s % kMmaStages, k0 = s * kBk;
-    const bool a_in = k0 + ac < kn;
-#pragma unroll
-    for (int q = 0; q < LA; ++q) {
-      const bool in = a_in && RA * q < rows_left;
-      cp_async8(&sm.As[buf][ar + RA * q][ac], in ? pa + k0 + q * stepa : g.a, in);
-    }
-#pragma unroll
-    for (int q = 0; q < LB; ++q) {
-      const bool in = b_in && k0 + br + RB * q < kn;
-      cp_async8(&sm.Bs[buf][br + RB * q][bc], in ? pb + k0 * r.ldb + q * stepb : g.b, in);
-    }
-  };
-  double acc[FM][FN][4];
-#pragma unroll
-  for (int i = 0; i < FM; ++i)
-#pragma unroll
-    for (int j = 0; j < FN; ++j)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.0;
-
-  pdl_wait();  // A may be the previous kernel's output
-#pragma unroll
-  for (int s = 0; s < kMmaStages - 1; ++s) {
-    if (s < nk) issue(s);
-    cp_async_commit();
-  }
-  const int wm = (warp >> 1) * WM, wn = (warp & 1) * WN, fr = lane >> 2, fk = lane & 3;
-  for (int s = 0; s < nk; ++s) {
-    cp_async_wait<kMmaStages - 2>();  // this thread's copies of slab s have landed
-    __syncthreads();                  // everyone's have, and slab s - 1 is consumed
-    if (s + kMmaStages - 1 < nk) issue(s + kMmaStages - 1);
-    cp_async_commit();
-    const int buf = s % kMmaStages;
-    const int steps = kn - s * kBk > 8 ? 2 : 1;  // (a last slab of up to eight takes one)
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      if (h < steps) {
-        double fa[FM][4], fb[FN][2];
-#pragma unroll
-        for (int i = 0; i < FM; ++i) {
-          const double* p = &sm.As[buf][wm + 16 * i + fr][8 * h + fk];
-          fa[i][0] = p[0];
-          fa[i][1] = p[8 * kMmaPadA];
-          fa[i][2] = p[4];
-          fa[i][3] = p[8 * kMmaPadA + 4];
-        }
-#pragma unroll
-        for (int j = 0; j < FN; ++j) {
-          const double* p = &sm.Bs[buf][8 * h + fk][wn + 8 * j + fr];
-          fb[j][0] = p[0];
-          fb[j][1] = p[4 * (TN + 4)];
-        }
-#pragma unroll
-        for (int i = 0; i < FM; ++i)
-#pragma unroll
-          for (int j = 0; j < FN; ++j) mma_f64(acc[i][j], fa[i], fb[j]);
-      }
-    }
-  }
-  cp_async_wait<0>();
-
-  // element e of fragment (i, j): row 16 i + fr + 8 (e / 2), column 8 j + 2 fk + e % 2
+  const int wm = (warp >> 1) * (TM / 2), wn = (warp & 1) * (TN / 2), fr = lane >> 2,
+            fk = lane & 3;
   if (r.splits > 1) {
     // split K: park this partial tile, and let the last of the tile's splits to arrive
     // sum all of them in split order (a fixed order, so the result is deterministic)
@@ -209,20 +116,151 @@ gemm_f64_kernel(const GemmArgs g) {
     }
     if (tid == 0) g.counters[r.cnt_off + t2] = 0u;  // leave the counters zero for the next run
   }
-  double* const pc = g.c + r.coff;
+  // through shared memory, so that a store instruction writes 32 consecutive columns of a row
+  // (a fragment holds pairs of columns of eight rows: stored directly, half of each 32-byte
+  // sector a time)
+  constexpr int kPitch = TN + 4;
+  static_assert(TM * kPitch <= kMmaStages * (TM * kMmaPadA + kBk * kPitch),
+                "the tile fits the drained slabs");
+  double* const stage = &sm.As[0][0][0];
+  __syncthreads();  // every warp is done with the last slab
 #pragma unroll
   for (int i = 0; i < FM; ++i)
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int64_t gm = m0 + wm + 16 * i + fr + 8 * h;
-      if (gm >= r.M) continue;
+    for (int h = 0; h < 2; ++h)
 #pragma unroll
-      for (int j = 0; j < FN; ++j) {
-        const int64_t gn = n0 + wn + 8 * j + 2 * fk;
-        if (gn < r.N) pc[gm * r.ldc + gn] = acc[i][j][2 * h];
-        if (gn + 1 < r.N) pc[gm * r.ldc + gn + 1] = acc[i][j][2 * h + 1];
+      for (int j = 0; j < FN; ++j)
+        *reinterpret_cast<double2*>(stage + (wm + 16 * i + fr + 8 * h) * kPitch + wn + 8 * j +
+                                    2 * fk) = make_double2(acc[i][j][2 * h], acc[i][j][2 * h + 1]);
+  __syncthreads();
+  double* const pc = g.c + r.coff + m0 * r.ldc + n0;
+  const int rows = static_cast<int>(min(r.M - m0, int64_t(TM)));
+  const int cols = static_cast<int>(min(r.N - n0, int64_t(TN)));
+  for (int row = warp; row < rows; row += kMmaThreads / 32)
+#pragma unroll
+    for (int c = 0; c < TN; c += 32)
+      if (c + lane < cols) pc[row * r.ldc + c + lane] = stage[row * kPitch + c + lane];
+}
+
+// One TM x TN output tile, or one K split of it, by a CTA of four warps in a 2 x 2 grid.
+template <int TM, int TN>
+__global__ void __launch_bounds__(kMmaThreads, (TM == 64 ? 3 : 6))
+gemm_f64_kernel(const GemmArgs g) {
+  extern __shared__ __align__(16) uint8_t gemm_smem[];
+  auto& sm = *reinterpret_cast<MmaSmem<TM, TN>*>(gemm_smem);
+  constexpr int WM = TM / 2, WN = TN / 2;        // a warp's part of the tile
+  constexpr int FM = WM / 16, FN = WN / 8;       // its m16 x n8 fragments
+  constexpr int LA = TM * kBk / kMmaThreads, LB = TN * kBk / kMmaThreads;
+  constexpr int RA = kMmaThreads / kBk, RB = kMmaThreads / TN;  // rows per round of copies
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t tile = blockIdx.x;
+  GemmRow r;
+  bool ok = load_row(g, tile, r);
+  ok = ok && footprint_ok(r, g.n_a, g.n_b, g.n_c);
+  if (ok && r.splits > 1) {
+    const int64_t nt = ((r.M + TM - 1) / TM) * r.tiles_n;
+    ok = r.ksplit > 0 && r.ksplit % kBk == 0 && r.cnt_off >= 0 && r.cnt_off + nt <= g.n_cnt &&
+         r.part_off >= 0 && r.part_off + nt * r.splits * TM * TN <= g.n_parts;
+  }
+  if (!ok) {
+    if (tid == 0) raise_bounds();
+    return;
+  }
+  // (a row's tiles are counted in 32 bits: the grid is; 64-bit divisions cost as much as the
+  // tile's multiply-adds)
+  const int64_t local = tile - r.tile_begin;
+  if (local < 0 || r.splits > INT32_MAX || r.tiles_n < 1 || r.tiles_n > INT32_MAX) {
+    if (tid == 0) raise_bounds();
+    return;
+  }
+  uint32_t t2 = static_cast<uint32_t>(local), split = 0;
+  if (r.splits > 1) {
+    split = t2 % static_cast<uint32_t>(r.splits);
+    t2 /= static_cast<uint32_t>(r.splits);
+  }
+  const uint32_t trow = t2 / static_cast<uint32_t>(r.tiles_n);
+  const int64_t m0 = static_cast<int64_t>(trow) * TM;
+  const int64_t n0 = static_cast<int64_t>(t2 - trow * static_cast<uint32_t>(r.tiles_n)) * TN;
+  if (m0 >= r.M || n0 >= r.N) return;
+  const int64_t kb = r.splits > 1 ? split * r.ksplit : 0;
+  const int64_t ke = r.splits > 1 ? min(r.K, kb + r.ksplit) : r.K;
+  const int kn = ke > kb ? static_cast<int>(min(ke - kb, int64_t(INT32_MAX - kBk))) : 0;
+  const int nk = (kn + kBk - 1) / kBk;
+
+  // this thread's copies: A element (ar + RA q, ac), B element (br + RB q, bc) of a slab
+  const int ar = tid / kBk, ac = tid % kBk, br = tid / TN, bc = tid % TN;
+  const double* const pa = g.a + r.aoff + (m0 + ar) * r.lda + kb + ac;
+  const double* const pb = g.b + r.boff + (kb + br) * r.ldb + n0 + bc;
+  const int64_t stepa = RA * r.lda, stepb = RB * r.ldb;
+  const int rows = static_cast<int>(min(r.M - m0, int64_t(TM)));
+  const int cols = static_cast<int>(min(r.N - n0, int64_t(TN)));
+  const int rows_left = rows - ar;
+  const bool b_in = bc < cols;
+  auto issue = [&](int s) {
+    const int buf = s % kMmaStages, k0 = s * kBk;
+    const bool a_in = k0 + ac < kn;
+#pragma unroll
+    for (int q = 0; q < LA; ++q) {
+      const bool in = a_in && RA * q < rows_left;
+      cp_async8(&sm.As[buf][ar + RA * q][ac], in ? pa + k0 + q * stepa : g.a, in);
+    }
+#pragma unroll
+    for (int q = 0; q < LB; ++q) {
+      const bool in = b_in && k0 + br + RB * q < kn;
+      cp_async8(&sm.Bs[buf][br + RB * q][bc], in ? pb + k0 * r.ldb + q * stepb : g.b, in);
+    }
+  };
+  double acc[FM][FN][4];
+#pragma unroll
+  for (int i = 0; i < FM; ++i)
+#pragma unroll
+    for (int j = 0; j < FN; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.0;
+
+  pdl_wait();  // A may be the previous kernel's output
+#pragma unroll
+  for (int s = 0; s < kMmaStages - 1; ++s) {
+    if (s < nk) issue(s);
+    cp_async_commit();
+  }
+  const int wm = (warp >> 1) * WM, wn = (warp & 1) * WN, fr = lane >> 2, fk = lane & 3;
+  for (int s = 0; s < nk; ++s) {
+    cp_async_wait<kMmaStages - 2>();  // this thread's copies of slab s have landed
+    __syncthreads();                  // everyone's have, and slab s - 1 is consumed
+    if (s + kMmaStages - 1 < nk) issue(s + kMmaStages - 1);
+    cp_async_commit();
+    const int buf = s % kMmaStages;
+    // (a last slab of up to eight takes one step, a warp past the tile's edge none)
+    const int steps = wm >= rows || wn >= cols ? 0 : (kn - s * kBk > 8 ? 2 : 1);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (h < steps) {
+        double fa[FM][4], fb[FN][2];
+#pragma unroll
+        for (int i = 0; i < FM; ++i) {
+          const double* p = &sm.As[buf][wm + 16 * i + fr][8 * h + fk];
+          fa[i][0] = p[0];
+          fa[i][1] = p[8 * kMmaPadA];
+          fa[i][2] = p[4];
+          fa[i][3] = p[8 * kMmaPadA + 4];
+        }
+#pragma unroll
+        for (int j = 0; j < FN; ++j) {
+          const double* p = &sm.Bs[buf][8 * h + fk][wn + 8 * j + fr];
+          fb[j][0] = p[0];
+          fb[j][1] = p[4 * (TN + 4)];
+        }
+#pragma unroll
+        for (int i = 0; i < FM; ++i)
+#pragma unroll
+          for (int j = 0; j < FN; ++j) mma_f64(acc[i][j], fa[i], fb[j]);
       }
     }
+  }
+  cp_async_wait<0>();
+
+  flush_tile<TM, TN>(g, r, t2, split, m0, n0, acc, sm);
 }
 
 template <int TM, int TN>

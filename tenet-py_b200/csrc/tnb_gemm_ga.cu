@@ -57,7 +57,9 @@ gemm_ga_kernel(const GaArgs ga) {
   const int tid = threadIdx.x;
   if (tid == 0) {
     GemmRow r;
-    bool ok = load_row(g.table, g.n_gemm, g.tile_map, blockIdx.x, r);
+    const int64_t row = g.tile_map[blockIdx.x];
+    bool ok = row >= 0 && row < g.n_gemm;
+    if (ok) read_row(g.table + row * TNB_GEMM_WIDTH, r);
     ok = ok && r.M >= 0 && r.N >= 0 && r.K >= 0 && r.K <= kGaMaxK && r.coff >= 0 &&
          (r.M == 0 || r.N == 0 || r.coff + (r.M - 1) * r.ldc + r.N <= g.n_c);
     if (ok && r.K > 0 && r.M > 0 && r.N > 0)

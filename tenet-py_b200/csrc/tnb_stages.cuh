@@ -568,25 +568,30 @@ struct GemmRow {
       part_off, cnt_off;
 };
 
-__device__ __forceinline__ bool load_row(const int64_t* __restrict__ table, int64_t n_gemm,
-                                         const int32_t* __restrict__ tile_map, int64_t tile,
-                                         GemmRow& r) {
-  const int64_t g = tile_map[tile];
-  if (g < 0 || g >= n_gemm) return false;
-  const int64_t* t = table + g * TNB_GEMM_WIDTH;
-  r.M = t[0]; r.N = t[1]; r.K = t[2]; r.aoff = t[3]; r.lda = t[4]; r.boff = t[5];
-  r.ldb = t[6]; r.coff = t[7]; r.ldc = t[8]; r.tile_begin = t[9]; r.tiles_n = t[10];
-  r.splits = t[12] > 1 ? t[12] : 1; r.ksplit = t[13]; r.part_off = t[14]; r.cnt_off = t[15];
-  return true;
+// A descriptor row's words, as eight 16-byte loads where the row is aligned for them.
+__device__ __forceinline__ void read_row(const int64_t* __restrict__ t, GemmRow& r) {
+  int64_t w[TNB_GEMM_WIDTH];
+  if ((reinterpret_cast<uintptr_t>(t) & 15) == 0) {
+#pragma unroll
+    for (int i = 0; i < TNB_GEMM_WIDTH; i += 2) {
+      const longlong2 v = __ldg(reinterpret_cast<const longlong2*>(t + i));
+      w[i] = v.x;
+      w[i + 1] = v.y;
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < TNB_GEMM_WIDTH; ++i) w[i] = __ldg(t + i);
+  }
+  r.M = w[0]; r.N = w[1]; r.K = w[2]; r.aoff = w[3]; r.lda = w[4]; r.boff = w[5];
+  r.ldb = w[6]; r.coff = w[7]; r.ldc = w[8]; r.tile_begin = w[9]; r.tiles_n = w[10];
+  r.splits = w[12] > 1 ? w[12] : 1; r.ksplit = w[13]; r.part_off = w[14]; r.cnt_off = w[15];
 }
 
 __device__ __forceinline__ bool load_row(const GemmArgs& g, int64_t tile, GemmRow& r) {
-  if (g.tile_rows == nullptr) return load_row(g.table, g.n_gemm, g.tile_map, tile, r);
-  if (tile < 0 || tile >= g.n_gemm) return false;  // n_gemm holds the tile count here
-  const int64_t* t = g.tile_rows + tile * TNB_GEMM_WIDTH;
-  r.M = t[0]; r.N = t[1]; r.K = t[2]; r.aoff = t[3]; r.lda = t[4]; r.boff = t[5];
-  r.ldb = t[6]; r.coff = t[7]; r.ldc = t[8]; r.tile_begin = t[9]; r.tiles_n = t[10];
-  r.splits = t[12] > 1 ? t[12] : 1; r.ksplit = t[13]; r.part_off = t[14]; r.cnt_off = t[15];
+  int64_t row = tile;
+  if (g.tile_rows == nullptr) row = g.tile_map[tile];
+  if (row < 0 || row >= g.n_gemm) return false;  // (n_gemm holds the tile count of tile rows)
+  read_row((g.tile_rows == nullptr ? g.table : g.tile_rows) + row * TNB_GEMM_WIDTH, r);
   return true;
 }
 
