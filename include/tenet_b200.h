@@ -610,6 +610,16 @@ int tnb_svd_compact(const int64_t* rows, int64_t n_rows, const double* u, int64_
 int tnb_block_lq(const int64_t* rows, int64_t n_rows, const double* b, int64_t n_b,
                  double* l, int64_t n_l, double* q, int64_t n_q, double* work, int64_t n_work,
                  int64_t smem_doubles, void* stream);
+/*
+ * The same factorisation with a sector's columns dealt to 32 warps that hand the reflectors
+ * on without CTA barriers (rows as above, w_off unused).  Takes sectors with nb <= max_nb <=
+ * 512 whose mb*nb + 3 min(mb, nb) doubles fit smem_doubles of shared memory.  Same factors
+ * and gauge as tnb_block_lq to rounding.
+ */
+int tnb_block_lq_warp(const int64_t* rows, int64_t n_rows, const double* b, int64_t n_b,
+                      double* l, int64_t n_l, double* q, int64_t n_q, int64_t max_nb,
+                      int64_t smem_doubles, void* stream);
+
 
 /* Library version (major*10000 + minor*100 + patch). */
 int tnb_version(void);

@@ -723,6 +723,199 @@ block_lq_kernel(const int64_t* __restrict__ rows, int64_t n_rows, const double* 
   }
 }
 
+// The same factorisation without CTA barriers, for sectors whose W fits shared memory (rows
+// of up to 512): 16 warps, column c of W belongs to warp c % 16.  A warp waits for reflector
+// j (an mbarrier each), applies it to its own later columns, and the owner of column j + 1
+// forms and publishes the next reflector before it turns to its other columns, so the steps'
+// only chain is: the wait, one column's dot product and update, its norm, the reflector's
+// scalars.  Reflectors stay in W below the diagonal; Q's columns are then formed one per warp
+// in registers (column c needs reflectors c..0 only).
+// What bounded block_lq_kernel: per reflector three CTA-wide barriers, a CTA-wide sum and a
+// round of column updates, from global memory where W and Q together do not fit (197 x 77).
+// Measured: seven sectors up to 77 x 197 in 195 us (688 before).  32 warps: 215, 24: 279 (the
+// column arithmetic); columns held in registers: 215-235, the selection of the next
+// reflector's column costs more than the shared-memory traffic it saves; waiting by polling a
+// counter instead of an mbarrier: 13 us more.
+constexpr int kLqThreads = 512, kLqWarps = kLqThreads / 32, kLqMaxRows = 512;
+constexpr long long kLqWaitCycles = 4000000000LL;  // ~2 s at the boost clock
+
+// Wait until the reflector whose mbarrier this is has been published; false when the wait
+// gives up.  (try_wait suspends the warp: 31 warps polling a counter took the shared-memory
+// slots that the working ones need.)
+__device__ __forceinline__ bool lq_wait(const double* mbar) {
+  const uint32_t p = static_cast<uint32_t>(__cvta_generic_to_shared(mbar));
+  const long long t0 = clock64();
+  while (true) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(done) : "r"(p) : "memory");
+    if (done) return true;
+    if (clock64() - t0 > kLqWaitCycles) return false;
+  }
+}
+
+template <int E>
+__global__ void __launch_bounds__(kLqThreads)
+block_lq_warp_kernel(const int64_t* __restrict__ rows, int64_t n_rows,
+                     const double* __restrict__ b, int64_t n_b, double* __restrict__ lout,
+                     int64_t n_l, double* __restrict__ qout, int64_t n_q,
+                     int64_t smem_doubles) {
+  extern __shared__ __align__(16) double qr_smem[];
+  const int64_t blk = blockIdx.x;
+  if (blk >= n_rows) return;
+  const int64_t* row = rows + blk * kQrRow;
+  const int64_t mb = row[0], nb = row[1], b_off = row[2], l_off = row[3], q_off = row[4];
+  const int64_t kk = mb < nb ? mb : nb;
+  const bool ok = mb >= 0 && nb >= 0 && nb <= 32 * E && mb <= smem_doubles && b_off >= 0 &&
+                  b_off + mb * nb <= n_b && l_off >= 0 && l_off + mb * kk <= n_l && q_off >= 0 &&
+                  q_off + kk * nb <= n_q && mb * nb + 3 * kk <= smem_doubles;
+  if (!ok) {
+    if (threadIdx.x == 0) raise_bounds();
+    return;
+  }
+  const int m = static_cast<int>(nb), n = static_cast<int>(mb), k = static_cast<int>(kk);
+  if (k == 0) return;
+  double* const W = qr_smem;  // column j (row j of B) at W + j * m
+  double* const tau = W + m * n;
+  double* const beta = tau + k;
+  double* const mbar = beta + k;  // one mbarrier per reflector
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int e = tid; e < m * n; e += kLqThreads) W[e] = __ldg(b + b_off + e);
+  for (int j = tid; j < k; j += kLqThreads)
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;"
+                 :: "r"(static_cast<uint32_t>(__cvta_generic_to_shared(mbar + j))) : "memory");
+  __syncthreads();
+
+  // reflector j of the up-to-date column j, by its owner: LAPACK's dlarfg with dlapy2's norm
+  auto reflect = [&](int j) {
+    double* const w = W + j * m;
+    double x2 = 0.0;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int i = lane + 32 * e;
+      const double x = i > j && i < m ? w[i] : 0.0;
+      x2 = fma(x, x, x2);
+    }
+    x2 = warp_sum(x2);
+    const double alpha = w[j];
+    double t = 0.0, bt = alpha, scale = 1.0;
+    if (x2 > 0.0) {
+      const double xnorm = sqrt(x2), aa = fabs(alpha);
+      const double big = fmax(aa, xnorm), z = fmin(aa, xnorm);
+      const double q = z / big;
+      const double nrm = z == 0.0 ? big : __dmul_rn(big, sqrt(__dadd_rn(1.0, __dmul_rn(q, q))));
+      bt = alpha >= 0.0 ? -nrm : nrm;
+      t = (bt - alpha) / bt;
+      scale = 1.0 / (alpha - bt);
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const int i = lane + 32 * e;
+        if (i > j && i < m) w[i] *= scale;
+      }
+    }
+    if (lane == 0) {
+      tau[j] = t;
+      beta[j] = bt;
+    }
+    __syncwarp();
+    if (lane == 0)
+      asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];"
+                   :: "r"(static_cast<uint32_t>(__cvta_generic_to_shared(mbar + j))) : "memory");
+  };
+  // reflector j, v = [0 .., 1 at j, w_j below], and H_j on column c
+  auto load = [&](int j, double (&v)[E]) {
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int i = lane + 32 * e;
+      v[e] = i > j && i < m ? W[j * m + i] : (i == j ? 1.0 : 0.0);
+    }
+  };
+  auto apply = [&](const double (&v)[E], int j, int c, double t) {
+    double* const w = W + c * m;
+    double x[E], d = 0.0;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int i = lane + 32 * e;
+      x[e] = i >= j && i < m ? w[i] : 0.0;
+      d = fma(v[e], x[e], d);
+    }
+    d = warp_sum(d) * t;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int i = lane + 32 * e;
+      if (i >= j && i < m) w[i] = fma(-d, v[e], x[e]);
+    }
+  };
+  bool dead = false;
+  if (warp == 0) reflect(0);
+  for (int j = 0; j < k; ++j) {
+    int c = warp;
+    if (c <= j) c += (j - c + kLqWarps) / kLqWarps * kLqWarps;  // the first own column past j
+    if (c >= n) break;  // nothing left to update
+    if (!dead && !lq_wait(mbar + j)) {
+      dead = true;  // go on without waiting: every warp reaches the barrier below
+      atomicCAS(&g_device_error, 0, TNB_ETIMEOUT);
+    }
+    __syncwarp();
+    const double t = tau[j];
+    double v[E];
+    load(j, v);
+    for (; c < n; c += kLqWarps) {
+      if (t != 0.0) apply(v, j, c, t);
+      __syncwarp();
+      if (c == j + 1 && c < k) reflect(c);
+    }
+  }
+  __syncthreads();
+
+  // L = R^T (mb x k): row i is column i of R, R[p][i] for p < i, beta on the diagonal
+  for (int i = warp; i < n; i += kLqWarps)
+    for (int p = lane; p < k; p += 32)
+      lout[l_off + static_cast<int64_t>(i) * k + p] =
+          p < i ? W[i * m + p] : (p == i ? beta[p] : 0.0);
+  // column c of Q = H_0 ... H_{k-1} [I; 0], from the last reflection that moves it back
+  for (int c = warp; c < k; c += kLqWarps) {
+    double x[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) x[e] = lane + 32 * e == c ? 1.0 : 0.0;
+    for (int j = c; j >= 0; --j) {
+      const double t = tau[j];
+      if (t == 0.0) continue;
+      double v[E], d = 0.0;
+      load(j, v);
+#pragma unroll
+      for (int e = 0; e < E; ++e) d = fma(v[e], x[e], d);
+      d = warp_sum(d) * t;
+#pragma unroll
+      for (int e = 0; e < E; ++e) x[e] = fma(-d, v[e], x[e]);
+    }
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int i = lane + 32 * e;
+      if (i < m) qout[q_off + static_cast<int64_t>(c) * m + i] = x[e];
+    }
+  }
+}
+
+template <int E>
+static cudaError_t launch_lq_warp(unsigned grid, int64_t smem_doubles, cudaStream_t s,
+                                  const int64_t* rows, int64_t n_rows, const double* b,
+                                  int64_t n_b, double* l, int64_t n_l, double* q, int64_t n_q) {
+  static PerDeviceOnce opted;
+  const cudaError_t e = opted.once([] {
+    return cudaFuncSetAttribute(block_lq_warp_kernel<E>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                static_cast<int>(kSvdSmemMaxBytes - 1024));
+  });
+  if (e != cudaSuccess) return e;
+  block_lq_warp_kernel<E><<<grid, kLqThreads, static_cast<size_t>(smem_doubles) * 8, s>>>(
+      rows, n_rows, b, n_b, l, n_l, q, n_q, smem_doubles);
+  return cudaSuccess;
+}
+
 static PerDeviceOnce g_lq_opt;
 
 }  // namespace tnb
@@ -749,4 +942,35 @@ extern "C" int tnb_block_lq(const int64_t* rows, int64_t n_rows, const double* b
                          static_cast<size_t>(smem_doubles) * 8, tnb::as_stream(stream)>>>(
       rows, n_rows, b, n_b, l, n_l, q, n_q, work, n_work, smem_doubles);
   return tnb::check_launch("tnb_block_lq");
+}
+
+extern "C" int tnb_block_lq_warp(const int64_t* rows, int64_t n_rows, const double* b,
+                                 int64_t n_b, double* l, int64_t n_l, double* q, int64_t n_q,
+                                 int64_t max_nb, int64_t smem_doubles, void* stream) {
+  TNB_REQUIRE(n_rows >= 0 && n_b >= 0 && n_l >= 0 && n_q >= 0, "tnb_block_lq_warp: negative size");
+  TNB_REQUIRE(smem_doubles >= 0 && smem_doubles <= tnb_block_svd_smem_doubles(),
+              "tnb_block_lq_warp: shared-memory request beyond the limit");
+  TNB_REQUIRE(max_nb >= 0 && max_nb <= tnb::kLqMaxRows,
+              "tnb_block_lq_warp: sectors of at most 512 columns");
+  if (n_rows == 0) return TNB_OK;
+  TNB_REQUIRE(rows && b && l && q, "tnb_block_lq_warp: null pointer");
+  TNB_REQUIRE(n_rows < (1ll << 31), "tnb_block_lq_warp: too many sectors");
+  const unsigned grid = static_cast<unsigned>(n_rows);
+  cudaStream_t s = tnb::as_stream(stream);
+  cudaError_t e;
+  if (max_nb <= 32)
+    e = tnb::launch_lq_warp<1>(grid, smem_doubles, s, rows, n_rows, b, n_b, l, n_l, q, n_q);
+  else if (max_nb <= 64)
+    e = tnb::launch_lq_warp<2>(grid, smem_doubles, s, rows, n_rows, b, n_b, l, n_l, q, n_q);
+  else if (max_nb <= 128)
+    e = tnb::launch_lq_warp<4>(grid, smem_doubles, s, rows, n_rows, b, n_b, l, n_l, q, n_q);
+  else if (max_nb <= 256)
+    e = tnb::launch_lq_warp<8>(grid, smem_doubles, s, rows, n_rows, b, n_b, l, n_l, q, n_q);
+  else
+    e = tnb::launch_lq_warp<16>(grid, smem_doubles, s, rows, n_rows, b, n_b, l, n_l, q, n_q);
+  if (e != cudaSuccess) {
+    tnb::set_error(std::string("tnb_block_lq_warp: ") + cudaGetErrorString(e));
+    return TNB_ECUDA;
+  }
+  return tnb::check_launch("tnb_block_lq_warp");
 }

@@ -380,20 +380,28 @@ class _LqPlan:
         ll, lq_ = matrix_layout(self.sl), matrix_layout(self.sq)
         self.n_l, self.n_q = ll.size, lq_.size
         smem_max = int(_lib.load().tnb_block_svd_smem_doubles())
-        rows, wo, smem = [], 0, 0
+        # the sectors of the warp kernel first (those that fit it), then the others
+        warp_rows, rows, wo = [], [], 0
+        self.smem = self.warp_smem = self.warp_nb = 0
         for c in sorted(ml.sectors):
             r, q = ml.shape[c]
             k = min(r, q)
             assert ll.shape[c] == (r, k) and lq_.shape[c] == (k, q)
+            head = (r, q, ml.base[c], ll.base[c], lq_.base[c])
+            if q <= 512 and r * q + 3 * k <= smem_max:
+                self.warp_smem = max(self.warp_smem, r * q + 3 * k)
+                self.warp_nb = max(self.warp_nb, q)
+                warp_rows.append((*head, -1, 0, 0))
+                continue
             need = q * r + q * k + 2 * k
             if need <= smem_max:
-                w = -1
-                smem = max(smem, need)
+                w, self.smem = -1, max(self.smem, need)
             else:
                 w, wo = wo, wo + need
-            rows.append((r, q, ml.base[c], ll.base[c], lq_.base[c], w, 0, 0))
-        self.n_rows, self.n_w, self.smem = len(rows), wo, smem
-        self.rows = torch.tensor(rows or [(0,) * 8], dtype=torch.int64, device=_exec.device())
+            rows.append((*head, w, 0, 0))
+        self.n_warp, self.n_rows, self.n_w = len(warp_rows), len(warp_rows) + len(rows), wo
+        self.rows = torch.tensor([*warp_rows, *rows] or [(0,) * 8], dtype=torch.int64,
+                                 device=_exec.device())
 
 
 @cache
@@ -424,9 +432,13 @@ def lq(t: SymmetricTensor, axes=None):
     qbuf = torch.empty(max(1, plan.n_q), **f64)
     work = torch.empty(max(1, plan.n_w), **f64)
     P = _exec.ptr
-    _lib.call("tnb_block_lq", P(plan.rows), plan.n_rows, P(buf), buf.numel(), P(lbuf),
-              lbuf.numel(), P(qbuf), qbuf.numel(), P(work), plan.n_w, plan.smem,
-              _exec.stream_ptr())
+    nw, st = plan.n_warp, _exec.stream_ptr()
+    if nw:
+        _lib.call("tnb_block_lq_warp", P(plan.rows), nw, P(buf), buf.numel(), P(lbuf),
+                  lbuf.numel(), P(qbuf), qbuf.numel(), plan.warp_nb, plan.warp_smem, st)
+    if nw < plan.n_rows:
+        _lib.call("tnb_block_lq", P(plan.rows) + 64 * nw, plan.n_rows - nw, P(buf), buf.numel(),
+                  P(lbuf), lbuf.numel(), P(qbuf), qbuf.numel(), P(work), plan.n_w, plan.smem, st)
     out_l, out_q = SymmetricTensor.empty(plan.sl), SymmetricTensor.empty(plan.sq)
     _raise_exec(plan.sl).run(lbuf, out_l.arena)
     _raise_exec(plan.sq).run(qbuf, out_q.arena)
