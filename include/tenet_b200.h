@@ -352,6 +352,16 @@ int64_t tnb_lanczos_step_max_n(void);
 int tnb_lanczos_step(int64_t n, double* w, const double* v, const double* vprev, double* vnext,
                      double* state, int32_t j, int32_t ncv, double tol, const int64_t* run_start,
                      const double* run_w, int64_t n_runs, void* stream);
+/*
+ * The same step on one thread-block cluster, for n up to tnb_lanczos_step_cluster_max_n()
+ * (131,072 doubles where a cluster of 16 CTAs can run); w is read only.  The sums are taken
+ * chunk by chunk, so they agree with tnb_lanczos_step's to rounding.
+ */
+int64_t tnb_lanczos_step_cluster_max_n(void);
+int tnb_lanczos_step_cluster(int64_t n, const double* w, const double* v, const double* vprev,
+                             double* vnext, double* state, int32_t j, int32_t ncv, double tol,
+                             const int64_t* run_start, const double* run_w, int64_t n_runs,
+                             void* stream);
 
 /*
  * FP64 reorthogonalisation for the precision form (no counterpart in the reference,

