@@ -27,8 +27,8 @@ namespace tnb {
 // pipe (8.5 of 9.2 TFLOP/s per scheduler over the chip), so four warps saturate an SM and
 // 56 of 64 issue slots stay free for the loads.  The 4 x 4 register tiles of DFMAs that ran
 // here took eight 64-bit shared loads per 16 multiply-adds and topped out at 14-16 TFLOP/s.
-// Measured on B200: 4096^3 32.3 TFLOP/s (16.4 with DFMA tiles; cuBLAS DGEMM 35.5), a dense
-// U(1) contraction's 1,466 tiles 28.0 (14.4), 3,520 products of about 108 x 82 x 24 8.7 (6.2,
+// Measured on B200: 4096^3 33.2 TFLOP/s (16.4 with DFMA tiles; cuBLAS DGEMM 35.5), a dense
+// U(1) contraction's 1,466 tiles 29.4 (14.4), 3,520 products of about 108 x 82 x 24 8.7 (6.2,
 // then bound by writing C), 95 MFLOP in 335 tiles 8.9 us (17.0).
 //
 // Each element's products are added in k order in one chain of fused multiply-adds, as
@@ -196,8 +196,8 @@ gemm_f64_kernel(const GemmArgs g) {
   const int cols = static_cast<int>(min(r.N - n0, int64_t(TN)));
   const int rows_left = rows - ar;
   const bool b_in = bc < cols;
-  auto issue = [&](int s) {
-    const int buf = s % kMmaStages, k0 = s * kBk;
+  auto issue = [&](int s, int buf) {
+    const int k0 = s * kBk;
     const bool a_in = k0 + ac < kn;
 #pragma unroll
     for (int q = 0; q < LA; ++q) {
@@ -221,42 +221,59 @@ gemm_f64_kernel(const GemmArgs g) {
   pdl_wait();  // A may be the previous kernel's output
 #pragma unroll
   for (int s = 0; s < kMmaStages - 1; ++s) {
-    if (s < nk) issue(s);
+    if (s < nk) issue(s, s);
     cp_async_commit();
   }
   const int wm = (warp >> 1) * WM, wn = (warp & 1) * WN, fr = lane >> 2, fk = lane & 3;
+  int buf = 0;
   for (int s = 0; s < nk; ++s) {
     cp_async_wait<kMmaStages - 2>();  // this thread's copies of slab s have landed
     __syncthreads();                  // everyone's have, and slab s - 1 is consumed
-    if (s + kMmaStages - 1 < nk) issue(s + kMmaStages - 1);
-    cp_async_commit();
-    const int buf = s % kMmaStages;
     // (a last slab of up to eight takes one step, a warp past the tile's edge none)
     const int steps = wm >= rows || wn >= cols ? 0 : (kn - s * kBk > 8 ? 2 : 1);
+    auto fragments = [&](int h, double (&fa)[FM][4], double (&fb)[FN][2]) {
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      if (h < steps) {
-        double fa[FM][4], fb[FN][2];
-#pragma unroll
-        for (int i = 0; i < FM; ++i) {
-          const double* p = &sm.As[buf][wm + 16 * i + fr][8 * h + fk];
-          fa[i][0] = p[0];
-          fa[i][1] = p[8 * kMmaPadA];
-          fa[i][2] = p[4];
-          fa[i][3] = p[8 * kMmaPadA + 4];
-        }
-#pragma unroll
-        for (int j = 0; j < FN; ++j) {
-          const double* p = &sm.Bs[buf][8 * h + fk][wn + 8 * j + fr];
-          fb[j][0] = p[0];
-          fb[j][1] = p[4 * (TN + 4)];
-        }
-#pragma unroll
-        for (int i = 0; i < FM; ++i)
-#pragma unroll
-          for (int j = 0; j < FN; ++j) mma_f64(acc[i][j], fa[i], fb[j]);
+      for (int i = 0; i < FM; ++i) {
+        const double* p = &sm.As[buf][wm + 16 * i + fr][8 * h + fk];
+        fa[i][0] = p[0];
+        fa[i][1] = p[8 * kMmaPadA];
+        fa[i][2] = p[4];
+        fa[i][3] = p[8 * kMmaPadA + 4];
       }
+#pragma unroll
+      for (int j = 0; j < FN; ++j) {
+        const double* p = &sm.Bs[buf][8 * h + fk][wn + 8 * j + fr];
+        fb[j][0] = p[0];
+        fb[j][1] = p[4 * (TN + 4)];
+      }
+    };
+    auto multiply = [&](const double (&fa)[FM][4], const double (&fb)[FN][2]) {
+#pragma unroll
+      for (int i = 0; i < FM; ++i)
+#pragma unroll
+        for (int j = 0; j < FN; ++j) mma_f64(acc[i][j], fa[i], fb[j]);
+    };
+    auto ahead = [&]() {
+      if (s + kMmaStages - 1 < nk) issue(s + kMmaStages - 1, buf == 0 ? kMmaStages - 1 : buf - 1);
+      cp_async_commit();
+    };
+    // 64-wide tiles issue the next slab's copies behind the first step's multiply-adds: with
+    // two or three warps on a scheduler the pipe would idle through that address arithmetic
+    // (dense 8 GF: 280 -> 273 us, 4096^3 32.6 -> 33.2 TFLOP/s). With up to six warps of
+    // 32-wide tiles another warp fills the gap and the earlier copy is worth more (512^3
+    // 18.8 us this way round, 21.7 the other).
+    double fa[FM][4], fb[FN][2];
+    if constexpr (TM == 32) ahead();
+    if (steps > 0) {
+      fragments(0, fa, fb);
+      multiply(fa, fb);
     }
+    if constexpr (TM == 64) ahead();
+    if (steps > 1) {
+      fragments(1, fa, fb);
+      multiply(fa, fb);
+    }
+    buf = buf + 1 == kMmaStages ? 0 : buf + 1;
   }
   cp_async_wait<0>();
 
