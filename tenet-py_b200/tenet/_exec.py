@@ -1186,19 +1186,42 @@ class GemmGroup:
         return q
 
 
-#: CTAs a composition's split-K tiles aim for (two per SM)
-SPLITK_TARGET_CTAS = 2 * N_SM
+#: per tile kind, in units of one contracted index of a lone tile (23 and 51 ns): what splitting
+#: along K costs (the partial sums' round trip and the tile counter), what each split adds, and
+#: how many times longer a tile takes with one, two, ... of them on its SM
+SPLIT_COST = {TILE_32: (110, 12, (1.0, 1.55, 2.2)), TILE_64: (60, 17, (1.0, 2.0))}
+#: splits per product at most
+SPLIT_MAX = 16
 
 
-def _splits(K: int, out_tiles_total: int) -> tuple[int, int]:
-    """K splits for a long-K product when the composition's output tiles cannot fill two
-    waves: (splits, ksplit) with ksplit a multiple of 16 and at least 32."""
-    if K <= 64 or out_tiles_total >= SPLITK_TARGET_CTAS:
-        return 1, 0
-    want = max(1, -(-SPLITK_TARGET_CTAS // max(out_tiles_total, 1)))
-    ks = max(32, -(-K // want))
-    ks = -(-ks // 16) * 16
-    return -(-K // ks), ks
+def _ksplit(products, kind: int) -> int:
+    """The K range of one split (a multiple of 16, at least 32) for a composition's FP64
+    tiles, or 0 to leave every product whole.
+
+    A lone tile is a serial chain over its longest K that leaves the other SMs idle and, 32
+    wide, half of its own: the range with the smallest sum of its own length, times the
+    crowding of the fullest SM if all work came in chains of that length, and the split's cost.
+    Measured in us, unsplit / this choice / two CTAs per SM with ranges >= 32 whatever that
+    costs (the choice before).  32-wide: three tiles, K = 96 3.4 / 3.4 / 4.9, K = 256
+    6.9 / 6.0 / 6.4, K = 1,024 23.7 / 8.5 / 9.0; 48 tiles, K = 192 5.8 / 5.8 / 7.3, K = 512
+    12.8 / 8.8 / 9.1; 180 tiles, K = 256 9.6 / 9.6 / 10.5, K = 1,024 33.2 / 25.2 / 25.2; 83
+    tiles, K = 37 to 785 19.1 / 13.4 / 13.4.  64-wide: 48 tiles, K = 128 8.7 / 8.7 / 15.1,
+    K = 512 28.5 / 17.5 / 30.2."""
+    cost, each, crowding = SPLIT_COST[kind]
+    K = max((p[2] for p in products), default=0)
+    work = sum(_tiles(p[0], p[1], kind)[0] * p[2] for p in products)
+    if K < 64 or work >= 2 * N_SM * K:
+        return 0
+    best, choice = crowding[-(-work // (N_SM * K)) - 1] * K, 0
+    for want in range(2, min(SPLIT_MAX, K // 32) + 1):
+        ks = max(32, -(-K // (16 * want)) * 16)
+        fullest = -(-work // (N_SM * ks))
+        if fullest > len(crowding):
+            break
+        took = crowding[fullest - 1] * ks + cost + each * -(-K // ks)
+        if took < best:
+            best, choice = took, ks
+    return choice
 
 
 def make_gemm(products, kind: int | None = None, split_k: bool = True) -> GemmTable:
@@ -1207,14 +1230,15 @@ def make_gemm(products, kind: int | None = None, split_k: bool = True) -> GemmTa
     if kind is None:
         kind = choose_kind(products)
     tw = 64 if kind == TILE_64 else 32  # split-K partial tile width (tiled FP64 kinds only)
-    out_total = sum(_tiles(p[0], p[1], kind)[0] for p in products)
+    ksplit = _ksplit(products, kind) if split_k and kind in (TILE_64, TILE_32) else 0
     rows = []
     tile = flops = n_cnt = n_parts = 0
     for M, N, K, ao, lda, bo, ldb, co, ldc in products:
         out_tiles, tn = _tiles(M, N, kind)
-        S, ks = (1, 0)
-        if split_k and kind in (TILE_64, TILE_32):
-            S, ks = _splits(K, out_total)
+        S, ks = 1, 0
+        if 0 < ksplit < K:  # in equal ranges
+            ks = -(-K // (16 * -(-K // ksplit))) * 16
+            S = -(-K // ks)
         row = [M, N, K, ao, lda, bo, ldb, co, ldc, tile, tn, out_tiles * S, 0, 0, 0, 0]
         if S > 1:
             row[12:16] = [S, ks, n_parts, n_cnt]
