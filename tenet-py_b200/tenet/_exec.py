@@ -205,10 +205,11 @@ class _UploadSlice:
         return self.up.ready()[self.lo:self.hi]
 
 
-def upload_together(tables, recorded: bool = False) -> None:
+def upload_together(tables, recorded: bool = False) -> Uploaded | None:
     """One upload (one staging copy, one device buffer, one event) for the arrays that every
     table in ``tables`` will read and that are not yet on the device, instead of one each
-    at its first run.  ``recorded``: the tables are about to be recorded into a sequence."""
+    at its first run.  ``recorded``: the tables are about to be recorded into a sequence.
+    Returns the upload, None when there was nothing to do."""
     todo, arrays = [], []
     for t in tables:
         if t is None:
@@ -219,10 +220,11 @@ def upload_together(tables, recorded: bool = False) -> None:
         todo.append((t, attr, len(arrays), len(arrays) + len(arrs)))
         arrays.extend(arrs)
     if not todo:
-        return
+        return None
     up = Uploaded(arrays)
     for t, attr, lo, hi in todo:
         setattr(t, attr, _UploadSlice(up, lo, hi))
+    return up
 
 
 class Uploaded:

@@ -417,6 +417,14 @@ class _BLink:
         self.direct, self.c_elems, self.deferred = direct, c_elems, False
 
 
+#: tiles of a product from which ``BatchedHeff2`` launches instead of replaying
+RECORD_MAX_TILES = 16 * _exec.N_SM
+
+#: addresses that stand for the input and output arenas in a recorded sequence (no buffer
+#: lies there; every replay substitutes the caller's)
+_X_SLOT, _Y_SLOT = 16, 32
+
+
 class BatchedHeff2:
     """The compiled two-site matvec (``program.heff2_program``: six launches in the FP64
     form) for ``n`` members at once: every table of the single-member chain replicated
@@ -484,6 +492,31 @@ class BatchedHeff2:
             else:
                 self.links[i + 1].a_g = pg
         self.flops = sum(bl.gemm.flops for bl in self.links)
+        self._record()
+
+    def _record(self) -> None:
+        """Record the launches for a replay by one library call: eight launches from Python
+        take the host about 54 us, the device 26 us at 32 members of the SU(2) chain's L = 64
+        bond.  A recorded product reads its descriptors through the tile map, 2-3% slower on
+        the device than one row per tile; from ``RECORD_MAX_TILES`` on the host is hidden and
+        the launches stay apart (us per run launched / recorded: 32 members 60 / 27, 128
+        members and 1,664 tiles 53 / 44, 256 members and 3,328 tiles 74 / 76).  So do products
+        on the tensor cores, whose operands are packed by a form that is not recorded."""
+        self._seq = None
+        parts = [p for bl in self.links if not bl.deferred for p in bl.gemm.parts]
+        if any(p.tiles >= RECORD_MAX_TILES or p.kind in (_exec.TILE_TC_TF32,
+                                                     _exec.TILE_TC_3XBF16)
+               for p in parts):
+            return
+        for p in parts:
+            p.work()  # zeroed before the upload's event, which other streams wait for
+        self._upload = _exec.upload_together(
+            [*(bl.a_g for bl in self.links), self.out_gather, *parts], recorded=True)
+        seq = _exec.Seq()
+        with seq:
+            self._launch(_exec._DevArray(_X_SLOT, self.n * self.in_size),
+                         _exec._DevArray(_Y_SLOT, self.n * self.out_size))
+        self._seq = seq
 
     @property
     def launches(self) -> int:
@@ -492,8 +525,20 @@ class BatchedHeff2:
                 + (self.out_gather is not None))
 
     def run(self, x: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
-        """``out[k] = H_k x[k]`` for the ``(n, size)`` arenas ``x`` and ``out``."""
-        src, pending = x.reshape(-1), None
+        """``out[k] = H_k x[k]`` for the ``(n, size)`` arenas ``x`` and ``out``.  The buffers
+        between the launches are this object's: it must not run on two streams at once."""
+        xs, ys = x.reshape(-1), out.reshape(-1)
+        if self._seq is not None and _exec._LOG is None and _exec.recording() is None \
+                and xs.numel() == self.n * self.in_size and ys.numel() == self.n * self.out_size:
+            if self._upload is not None:
+                self._upload.ready()
+            self._seq.run({_X_SLOT: xs.data_ptr(), _Y_SLOT: ys.data_ptr()})
+        else:
+            self._launch(xs, ys)
+        return out
+
+    def _launch(self, x, out) -> None:
+        src, pending = x, None
         for bl in self.links:
             ab, bb, cb = bl.bufs
             a = src if bl.direct else ab
@@ -507,10 +552,9 @@ class BatchedHeff2:
                 bl.gemm.run(a, bb, cb)
             src = cb
         if isinstance(self.out_gather, _exec.ProductGather):
-            self.out_gather.run(*pending, out.reshape(-1))
+            self.out_gather.run(*pending, out)
         elif self.out_gather is not None:
-            self.out_gather.run(src, out.reshape(-1))
-        return out
+            self.out_gather.run(src, out)
 
     def __call__(self, aa: TensorBatch) -> TensorBatch:
         if aa.structure != self.in_struct or aa.n != self.n:
