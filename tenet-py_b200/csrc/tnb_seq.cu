@@ -12,6 +12,7 @@
 #include <string>
 #include <vector>
 
+#include "tnb_lanczos_small.cuh"
 #include "tnb_stages.cuh"
 
 namespace tnb {
@@ -632,6 +633,144 @@ extern "C" int tnb_seq_run(const tnb_seq* s, int32_t n_patch, const void* const*
     if (rc_ != TNB_OK) return rc_; \
   } while (0)
 
+namespace tnb {
+namespace {
+
+// A matvec small enough for tnb_lanczos_small.cu: gathers from warp items and FP64 GEMMs
+// without split sums, every buffer, row and record in shared memory.  That holds bonds up to
+// some 420 elements a vector; there the one launch still takes 185 us where the launches take
+// 465 (134 elements 107 / 382, 26 elements 92 / 341, SU(2) chain, 20 vectors), so the
+// multiply-adds of a stage, at most sqrt(|A| |B| |C|) by Hoelder's inequality, and the mean
+// length of its sums, sqrt(|A| |B| / |C|), which one thread adds alone, are only held near what
+// was measured (36,700 and 87).  Fills `a` and returns the shared memory it takes, 0 if it does
+// not fit.
+constexpr double kSmallWork = 49152;
+constexpr double kSmallLength = 192;
+constexpr int64_t kSmallMaxN = 2048;
+
+int64_t plan_small(const tnb_seq* s, const void* x_slot, const void* y_slot, int64_t n,
+                   int64_t n_runs, SmallArgs* a) {
+  if (n > kSmallMaxN || s->ops.empty() || s->ops.size() > kSmallMaxStages || x_slot == y_slot)
+    return 0;
+  struct Buf {
+    int64_t at, n, off;
+  };
+  Buf bufs[kSmallMaxBufs];
+  int nb = 0;
+  auto add = [&](int64_t at, int64_t len) {  // its index, -1 when it does not fit
+    if (len < 0 || len > kSmallMaxSmem / 8 || (at == 0 && len > 0)) return -1;
+    for (int i = 0; i < nb; ++i)
+      if (bufs[i].at == at) {
+        if (bufs[i].n < len) bufs[i].n = len;
+        return i;
+      }
+    if (nb == kSmallMaxBufs) return -1;
+    bufs[nb] = {at, len, 0};
+    return nb++;
+  };
+  const int ix = add(as_word(x_slot), n), iy = add(as_word(y_slot), n);
+  if (ix < 0 || iy < 0) return 0;
+  int at[kSmallMaxStages][3];
+  int64_t rows_bytes = 0;
+  a->n_stages = static_cast<int>(s->ops.size());
+  for (int i = 0; i < a->n_stages; ++i) {
+    const tnb_seq::Op& op = s->ops[i];
+    const int64_t* w = op.w;
+    SmallStage& st = a->st[i];
+    st = SmallStage{};
+    if (op.code == kOpGatherItems) {
+      if (w[11] != 0 || w[13] != 0 || w[2] > kSmallMaxRows || (w[1] != 32 && w[1] != 64))
+        return 0;
+      st.gather = 1;
+      st.width = static_cast<int>(w[1]);
+      st.count = static_cast<int>(w[2]);
+      st.rows = as_ptr(w[0]);
+      st.term_src = static_cast<const int64_t*>(as_ptr(w[3]));
+      st.term_coeff = static_cast<const double*>(as_ptr(w[4]));
+      st.term_ld = static_cast<const int64_t*>(as_ptr(w[5]));
+      st.n_term = w[6];
+      at[i][0] = add(w[7], w[8]);
+      at[i][1] = -2;
+      at[i][2] = add(w[9], w[10]);
+      rows_bytes += 4 * static_cast<int64_t>(st.width) * st.count + 24 * w[10] + 48;
+    } else if (op.code == kOpGemm) {
+      if (w[4] != TNB_TILE_64 && w[4] != TNB_TILE_32 && w[4] != TNB_TILE_SKINNY &&
+          w[4] != TNB_TILE_WIDE)
+        return 0;
+      const double na = static_cast<double>(w[6]), nbb = static_cast<double>(w[8]),
+                   nc = static_cast<double>(w[10]);
+      if (w[1] > kSmallMaxRows || w[13] != 0 || na * nbb * nc > kSmallWork * kSmallWork ||
+          na * nbb > kSmallLength * kSmallLength * nc)
+        return 0;
+      st.count = static_cast<int>(w[1]);
+      st.rows = as_ptr(w[0]);
+      at[i][0] = add(w[5], w[6]);
+      at[i][1] = add(w[7], w[8]);
+      at[i][2] = add(w[9], w[10]);
+      rows_bytes += 16 * w[10] + 16;
+    } else {
+      return 0;
+    }
+    if (at[i][0] == -1 || at[i][1] == -1 || at[i][2] == -1 || at[i][0] == at[i][2] ||
+        at[i][1] == at[i][2] || at[i][2] == ix)
+      return 0;
+  }
+  if (bufs[ix].n != n || bufs[iy].n != n) return 0;
+  // buffers that share memory keep to the launches
+  int64_t off = 0;
+  for (int i = 0; i < nb; ++i) {
+    for (int k = 0; k < i; ++k)
+      if (bufs[i].at < bufs[k].at + 8 * bufs[k].n && bufs[k].at < bufs[i].at + 8 * bufs[i].n)
+        return 0;
+    bufs[i].off = off;
+    off += bufs[i].n;
+  }
+  const int64_t prev = off;
+  const int64_t weight = off + n;
+  off = (off + 2 * n + 1) / 2 * 2;  // rows and records start at a multiple of 16 bytes
+  if (8 * off + rows_bytes + 2 * n > kSmallMaxSmem) return 0;
+  int64_t byte = 8 * off;
+  for (int i = 0; i < a->n_stages; ++i) {
+    SmallStage& st = a->st[i];
+    auto take = [&](int64_t n_bytes) {
+      const int64_t from = byte;
+      byte += (n_bytes + 15) / 16 * 16;
+      return static_cast<int>(from);
+    };
+    const int64_t elems = s->ops[i].w[10];
+    st.rows_at = take(st.gather ? 4 * static_cast<int64_t>(st.width) * st.count : 0);
+    st.recs_at = take(16 * elems);
+    st.split_at = take(st.gather && st.width == 64 ? 8 * elems : 0);
+    const Buf& src = bufs[at[i][0]];
+    const Buf& dst = bufs[at[i][2]];
+    const int64_t* w = s->ops[i].w;
+    st.src = static_cast<int>(src.off);
+    st.n_src = static_cast<int>(st.gather ? w[8] : w[6]);
+    st.dst = static_cast<int>(dst.off);
+    st.n_dst = static_cast<int>(w[10]);
+    if (!st.gather) {
+      st.b = static_cast<int>(bufs[at[i][1]].off);
+      st.n_b = static_cast<int>(w[8]);
+    }
+  }
+  a->weight = static_cast<int>(weight);
+  a->order_at = static_cast<int>(byte);
+  a->n_bufs = 0;
+  for (int i = 0; i < nb; ++i)
+    if (i != ix && i != iy && bufs[i].n > 0)
+      a->buf[a->n_bufs++] = {static_cast<const double*>(as_ptr(bufs[i].at)),
+                             static_cast<int>(bufs[i].off), static_cast<int>(bufs[i].n)};
+  a->x = static_cast<int>(bufs[ix].off);
+  a->y = static_cast<int>(bufs[iy].off);
+  a->prev = static_cast<int>(prev);
+  a->n_runs = static_cast<int>(n_runs);
+  a->n = static_cast<int>(n);
+  return byte + 2 * n;
+}
+
+}  // namespace
+}  // namespace tnb
+
 extern "C" int tnb_lanczos_solve(const tnb_seq* matvec, const void* x_slot, const void* y_slot,
                                  int64_t n, int32_t ncv, double tol, int32_t reorth,
                                  const double* x0, double* v, int64_t ldv, double* w,
@@ -645,6 +784,23 @@ extern "C" int tnb_lanczos_solve(const tnb_seq* matvec, const void* x_slot, cons
               "tnb_lanczos_solve: null buffer");
   TNB_REQUIRE(!reorth || (vptrs && gs && multi_work), "tnb_lanczos_solve: reorth buffers");
   cudaStream_t s = tnb::as_stream(stream);
+  tnb::SmallArgs small;
+  const int64_t small_smem =
+      !reorth && n_runs > 0 && n_runs <= tnb::kSmallMaxRows
+          ? tnb::plan_small(matvec, x_slot, y_slot, n, n_runs, &small) : 0;
+  if (small_smem > 0) {
+    small.ncv = ncv;
+    small.tol = tol;
+    small.run_start = run_start;
+    small.run_w = run_w;
+    small.x0 = x0;
+    small.v = v;
+    small.ldv = ldv;
+    small.w = w;
+    small.state = state;
+    small.scal = scal;
+    return tnb::launch_lanczos_small(small, static_cast<int>(small_smem), s);
+  }
   cudaError_t e = cudaMemsetAsync(state, 0, sizeof(double) * (3 * ncv + 2), s);
   if (e != cudaSuccess) {
     tnb::set_error(std::string("tnb_lanczos_solve: ") + cudaGetErrorString(e));
