@@ -484,6 +484,11 @@ int tnb_seq_run(const tnb_seq* s, int32_t n_patch, const void* const* from, void
  * array of the ncv row pointers of v, gs = ncv doubles, multi_work of
  * tnb_multi_dot_work_bytes(n, ncv) bytes), ||w||^2 and tnb_lanczos_next.  `v` holds
  * ncv + 1 rows of stride ldv >= n; `scal` 2 doubles; dot_work tnb_dot_work_bytes(n).
+ * Without reorthogonalisation the vector work of a step is one launch up to
+ * tnb_lanczos_step_cluster_max_n() doubles, and a matvec of recorded gather items and FP64
+ * GEMMs without split sums whose buffers, rows and records fit one SM's shared memory (214
+ * KB; some 420 elements of an SU(2) chain) makes the whole solve one launch of one CTA, with
+ * the same bits; the recorded buffers between its stages are then read and not written.
  * The caller reads `state` (one synchronising copy), solves the tridiagonal, and calls
  * tnb_lanczos_ritz: out = normalised sum_j coef[j] v_j, and, when `correct` is given
  * (the FP64 sequence of the precision form), scal[1] = <out, H out> with H out in w2.

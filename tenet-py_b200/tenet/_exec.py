@@ -562,8 +562,8 @@ class GatherTable:
 #: run gathers of at least DIRECT_MIN_CHUNKS chunks from warp items
 #: (``tnb_block_gather_items``) where the table fits them (rank <= 4, 32-bit offsets within
 #: a segment), else from per-chunk rows (``tnb_block_gather_direct``).  Items win at every
-#: size: config-3's batched gathers 5.5 TB/s against 1.6 (439 against 1446 us in all), a
-#: 974-element one 1.3 against 1.8 us
+#: size: the gathers of a batched U(1) x U(1) x fZ2 update 5.5 TB/s against 1.6 (439 against
+#: 1446 us in all), a 974-element one 1.3 against 1.8 us
 DIRECT_GATHER = True
 DIRECT_MIN_CHUNKS = 0
 #: record the gathers of compiled chains as warp items too (a matvec on 256 multiplets 36.7

@@ -207,8 +207,8 @@ def svd_truncated(t: SymmetricTensor, axes=None, *, max_bond=None, cutoff=None,
     """``U, S, Vh`` on the truncated bond.  Same legs, keep rule and refusals as the
     reference; returns ``(U, S, Vh)``.  ``budget`` as in ``decide``.
 
-    All on the device: the lowering gather, one blockwise SVD launch (a CTA per coupled
-    sector), the decision launch (global order, cutoff prefix, budget walk), one read-back
+    All on the device: the lowering gather, the blockwise SVD (a cluster or a CTA per
+    coupled sector), the decision launch (global order, cutoff prefix, budget walk), one read-back
     of the decision, and one launch that packs the kept prefixes before the three raising
     gathers."""
     return svd_truncated_selected(t, axes, max_bond=max_bond, cutoff=cutoff,

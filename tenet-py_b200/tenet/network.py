@@ -261,9 +261,10 @@ class DeviceLanczos:
 
     def launch(self, x: torch.Tensor) -> None:
         """Enqueue the recurrence from start vector ``x`` (an arena of ``n`` doubles).  The
-        first call launches its ~9 ncv kernels one by one; from the second on, the whole
-        solve -- every buffer it touches is this solver's own and fixed -- is one graph
-        launch after a copy of ``x`` into the solver's start buffer."""
+        first call launches its kernels one by one (one for a small chain, else about six a
+        step); with ``GRAPH``, from the second on the whole solve -- every buffer it touches
+        is this solver's own and fixed -- is one graph launch after a copy of ``x`` into the
+        solver's start buffer."""
         if not (self.GRAPH and self._uses) or self._graph is False:
             self._uses += 1
             self._solve_call(x)
