@@ -128,6 +128,7 @@ class ContractionExec:
     pack: _exec.GatherTable
     gemm: _exec.GemmTable
     unpack: _exec.GatherTable
+    uploaded: bool = False  # (a table that changes its form uploads itself at its next run)
 
     def run(self, a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None,
             scratch: tuple | None = None) -> torch.Tensor:
@@ -140,9 +141,10 @@ class ContractionExec:
             ap, bp, cp = scratch
         if out is None:
             out = torch.empty(layout(self.out).size, dtype=torch.float64, device=dev)
-        if self.pack._dev is None:  # first run: every table of this contraction at once
+        if not self.uploaded:  # first run: every table of this contraction at once
             _exec.upload_together((self.pack, *getattr(self.gemm, "parts", (self.gemm,)),
                                    self.unpack))
+            self.uploaded = True
         self.pack.run(a, ap, b, bp)
         self.gemm.run(ap, bp, cp)
         self.unpack.run(cp, out)
