@@ -487,7 +487,7 @@ int tnb_seq_run(const tnb_seq* s, int32_t n_patch, const void* const* from, void
  * Without reorthogonalisation the vector work of a step is one launch up to
  * tnb_lanczos_step_cluster_max_n() doubles, and a matvec of recorded gather items and FP64
  * GEMMs without split sums whose buffers, rows and records fit one SM's shared memory (214
- * KB; some 420 elements of an SU(2) chain) makes the whole solve one launch of one CTA, with
+ * KB; some 620 elements of an SU(2) chain) makes the whole solve one launch of one CTA, with
  * the same bits; the recorded buffers between its stages are then read and not written.
  * The caller reads `state` (one synchronising copy), solves the tridiagonal, and calls
  * tnb_lanczos_ritz: out = normalised sum_j coef[j] v_j, and, when `correct` is given

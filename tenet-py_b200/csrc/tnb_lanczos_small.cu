@@ -15,8 +15,8 @@
 // offsets, with every check of the launched stages made there: decoding the items in every step
 // took 2,100 to 9,000 clocks a gather, a solve at 194 elements 305 us.
 //
-// Measured on B200, 20 vectors, from the call to the result: 26 elements 365 -> 108 us, 134
-// elements 399 -> 124, 420 elements 477 -> 199; a 16-site sweep 28.8 -> 20.8 ms.
+// Measured on B200, 20 vectors, from the call to the result: 26 elements 365 -> 111 us, 134
+// elements 399 -> 128, 420 elements 477 -> 203, 617 elements 482 -> 277; a 16-site sweep 28.8 -> 20.8 ms.
 //
 // Same arithmetic as the launches it replaces, in the same order (an element of a product as one
 // chain of fused multiply-adds over k, gathers in table order, the recurrence rounded operation
@@ -92,7 +92,7 @@ __device__ bool item_ok(const SmallStage& st, const int* row) {
   if (rank < 1 || rank > kItemMaxRank || ((row[10] >> 8) & 1) || n <= 0 || n > kItemMax ||
       base < 0 || row[6] < 0 || row[7] < row[6] || row[7] > st.n_term)
     return false;
-  int64_t total = 1, lo = item_i64(row[0], row[1]), hi = lo;
+  int64_t total = 1, lo = item_i64(row[0], row[1]), hi = lo, rr = 0, cc = 0;
   for (int d = 0; d < rank; ++d) {
     if (row[12 + d] <= 0) return false;
     total *= row[12 + d];
@@ -100,8 +100,11 @@ __device__ bool item_ok(const SmallStage& st, const int* row) {
     const int64_t x = static_cast<int64_t>(row[12 + d] - 1) * row[20 + d];
     lo += x < 0 ? x : 0;
     hi += x > 0 ? x : 0;
+    if (row[24 + d] < 0 || row[28 + d] < 0) return false;
+    rr += static_cast<int64_t>(row[12 + d] - 1) * row[24 + d];
+    cc += static_cast<int64_t>(row[12 + d] - 1) * row[28 + d];
   }
-  if (base + n > total || lo < 0 || hi >= st.n_dst) return false;
+  if (base + n > total || lo < 0 || hi >= st.n_dst || rr > 65535 || cc > 65535) return false;
   for (int i = 0; i < row[7] - row[6]; ++i) {
     int64_t ts;
     double cf;
@@ -120,18 +123,17 @@ __device__ bool item_ok(const SmallStage& st, const int* row) {
 }
 
 // A gathered element: its offset in shared memory and its first term's, how many terms and whose
-// item; the first coefficient.  Offsets fit 16 bits (kSmallMaxSmem).
-struct __align__(16) SmallMove {
-  uint16_t dst, src;
-  uint16_t terms, item;
-  double cf;
+// item.  Offsets fit 16 bits (kSmallMaxSmem); eight bytes an element and four more for several
+// terms, with coefficients and lengths left in the rows, reach 617 elements a vector where
+// records that held them too ended at 420.
+struct __align__(8) SmallMove {
+  uint16_t dst, src, terms, item;
 };
-// An element of a product: where its row of A, its column of B and itself lie.
-struct __align__(16) SmallDot {
-  uint16_t a, b, dst, k;
-  int ldb, pad;
+// An element of a product: where its row of A, its column of B and itself lie, and its row.
+struct __align__(8) SmallDot {
+  uint16_t a, b, dst, row;
 };
-static_assert(sizeof(SmallMove) == 16 && sizeof(SmallDot) == 16, "records of 16 bytes");
+static_assert(sizeof(SmallMove) == 8 && sizeof(SmallDot) == 8, "records of 8 bytes");
 
 __global__ void __launch_bounds__(kSmallThreads, 1)
 lanczos_small_kernel(const __grid_constant__ SmallArgs g) {
@@ -243,7 +245,7 @@ lanczos_small_kernel(const __grid_constant__ SmallArgs g) {
       if (st.gather) {
         const int* row = reinterpret_cast<const int*>(small_smem + st.rows_at) + k * st.width;
         SmallMove* const rec = reinterpret_cast<SmallMove*>(small_smem + st.recs_at) + at;
-        int2* const split = reinterpret_cast<int2*>(small_smem + st.split_at) + at;
+        ushort2* const split = reinterpret_cast<ushort2*>(small_smem + st.split_at) + at;
         const int rank = row[10] & 255, terms = row[7] - row[6];
         for (int q = lane; q < row[9]; q += 32) {
           int rem = row[8] + q, rr = 0, cc = 0, to = row[0];
@@ -260,23 +262,23 @@ lanczos_small_kernel(const __grid_constant__ SmallArgs g) {
           m.src = static_cast<uint16_t>(terms > 0 ? st.src + row[2] + row[11] * rr + cc : st.dst);
           m.terms = static_cast<uint16_t>(terms);
           m.item = static_cast<uint16_t>(k);
-          m.cf = __hiloint2double(row[5], row[4]);
           rec[q] = m;
-          if (st.width == 64) split[q] = make_int2(rr, cc);
+          if (st.width == 64) split[q] = make_ushort2(rr, cc);
         }
       } else {
         const int64_t* t = static_cast<const int64_t*>(st.rows) + k * TNB_GEMM_WIDTH;
         const int M = static_cast<int>(t[0]), N = static_cast<int>(t[1]), K = static_cast<int>(t[2]);
         SmallDot* const rec = reinterpret_cast<SmallDot*>(small_smem + st.recs_at) + at;
+        if (lane == 0)
+          reinterpret_cast<int2*>(small_smem + st.rows_at)[k] =
+              make_int2(K, K > 1 ? static_cast<int>(t[6]) : 0);
         for (int q = lane; q < M * N; q += 32) {
           const int m = q / N, c = q - m * N;
           SmallDot d;
           d.a = static_cast<uint16_t>(K > 0 ? st.src + t[3] + m * t[4] : 0);
           d.b = static_cast<uint16_t>(K > 0 ? st.b + t[5] + c : 0);
           d.dst = static_cast<uint16_t>(st.dst + t[7] + m * t[8] + c);
-          d.k = static_cast<uint16_t>(K);
-          d.ldb = K > 1 ? static_cast<int>(t[6]) : 0;
-          d.pad = 0;
+          d.row = static_cast<uint16_t>(k);
           rec[q] = d;
         }
       }
@@ -304,10 +306,10 @@ lanczos_small_kernel(const __grid_constant__ SmallArgs g) {
         const SmallMove* rec = reinterpret_cast<const SmallMove*>(small_smem + st.recs_at);
         for (int e = tid; e < total; e += kSmallThreads) {
           const SmallMove m = rec[e];
-          double acc = m.terms > 0 ? fma(m.cf, sm[m.src], 0.0) : 0.0;
+          const int* row = reinterpret_cast<const int*>(small_smem + st.rows_at) + m.item * st.width;
+          double acc = m.terms > 0 ? fma(__hiloint2double(row[5], row[4]), sm[m.src], 0.0) : 0.0;
           if (m.terms > 1) {
-            const int2 at = reinterpret_cast<const int2*>(small_smem + st.split_at)[e];
-            const int* row = reinterpret_cast<const int*>(small_smem + st.rows_at) + m.item * st.width;
+            const ushort2 at = reinterpret_cast<const ushort2*>(small_smem + st.split_at)[e];
 #pragma unroll 2
             for (int i = 1; i < m.terms; ++i) {
               int64_t ts;
@@ -323,11 +325,12 @@ lanczos_small_kernel(const __grid_constant__ SmallArgs g) {
         const SmallDot* rec = reinterpret_cast<const SmallDot*>(small_smem + st.recs_at);
         for (int e = tid; e < total; e += kSmallThreads) {
           const SmallDot d = rec[e];
+          const int2 len = reinterpret_cast<const int2*>(small_smem + st.rows_at)[d.row];
           const double* pa = sm + d.a;
           const double* pb = sm + d.b;
           double acc = 0.0;
 #pragma unroll 8
-          for (int i = 0; i < d.k; ++i, pb += d.ldb) acc = fma(pa[i], *pb, acc);
+          for (int i = 0; i < len.x; ++i, pb += len.y) acc = fma(pa[i], *pb, acc);
           sm[d.dst] = acc;
         }
       }

@@ -13,9 +13,9 @@ constexpr int kSmallMaxSmem = 214 * 1024;  // (and 12.5 KB of the kernel's own)
 struct SmallStage {
   int gather;           // 1: a gather of warp items, 0: a grouped GEMM
   int width, count;     // words per item row and items; or the GEMM table's rows in `count`
-  int rows_at;          // where a gather's item rows lie (bytes)
-  int recs_at;          // the records of the stage's elements, 16 bytes each (bytes)
-  int split_at;         // two words more per element of a gather of several terms (bytes)
+  int rows_at;          // where a gather's item rows, or K and ldb per GEMM row, lie (bytes)
+  int recs_at;          // the records of the stage's elements, 8 bytes each (bytes)
+  int split_at;         // four bytes more per element of a gather of several terms (bytes)
   int src, n_src;       // the gather's source, or A
   int b, n_b;           // B
   int dst, n_dst;

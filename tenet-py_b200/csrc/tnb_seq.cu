@@ -638,13 +638,13 @@ namespace {
 
 // A matvec small enough for tnb_lanczos_small.cu: gathers from warp items and FP64 GEMMs
 // without split sums, every buffer, row and record in shared memory.  That holds bonds up to
-// some 420 elements a vector; there the one launch still takes 185 us where the launches take
-// 465 (134 elements 107 / 382, 26 elements 92 / 341, SU(2) chain, 20 vectors), so the
-// multiply-adds of a stage, at most sqrt(|A| |B| |C|) by Hoelder's inequality, and the mean
-// length of its sums, sqrt(|A| |B| / |C|), which one thread adds alone, are only held near what
-// was measured (36,700 and 87).  Fills `a` and returns the shared memory it takes, 0 if it does
-// not fit.
-constexpr double kSmallWork = 49152;
+// some 620 elements a vector; there the one launch still takes 262 us where the launches take
+// 466 (420 elements 189 / 465, 134 elements 111 / 382, 26 elements 95 / 341, SU(2) chain, 20
+// vectors), so the multiply-adds of a stage, at most sqrt(|A| |B| |C|) by Hoelder's
+// inequality, and the mean length of its sums, sqrt(|A| |B| / |C|), which one thread adds
+// alone, are only held near what was measured (65,400 and 103).  Fills `a` and returns the
+// shared memory it takes, 0 if it does not fit.
+constexpr double kSmallWork = 98304;
 constexpr double kSmallLength = 192;
 constexpr int64_t kSmallMaxN = 2048;
 
@@ -692,7 +692,7 @@ int64_t plan_small(const tnb_seq* s, const void* x_slot, const void* y_slot, int
       at[i][0] = add(w[7], w[8]);
       at[i][1] = -2;
       at[i][2] = add(w[9], w[10]);
-      rows_bytes += 4 * static_cast<int64_t>(st.width) * st.count + 24 * w[10] + 48;
+      rows_bytes += 4 * static_cast<int64_t>(st.width) * st.count + 12 * w[10] + 48;
     } else if (op.code == kOpGemm) {
       if (w[4] != TNB_TILE_64 && w[4] != TNB_TILE_32 && w[4] != TNB_TILE_SKINNY &&
           w[4] != TNB_TILE_WIDE)
@@ -707,7 +707,7 @@ int64_t plan_small(const tnb_seq* s, const void* x_slot, const void* y_slot, int
       at[i][0] = add(w[5], w[6]);
       at[i][1] = add(w[7], w[8]);
       at[i][2] = add(w[9], w[10]);
-      rows_bytes += 16 * w[10] + 16;
+      rows_bytes += 8 * (w[10] + w[1]) + 32;
     } else {
       return 0;
     }
@@ -738,9 +738,9 @@ int64_t plan_small(const tnb_seq* s, const void* x_slot, const void* y_slot, int
       return static_cast<int>(from);
     };
     const int64_t elems = s->ops[i].w[10];
-    st.rows_at = take(st.gather ? 4 * static_cast<int64_t>(st.width) * st.count : 0);
-    st.recs_at = take(16 * elems);
-    st.split_at = take(st.gather && st.width == 64 ? 8 * elems : 0);
+    st.rows_at = take((st.gather ? 4 * static_cast<int64_t>(st.width) : 8) * st.count);
+    st.recs_at = take(8 * elems);
+    st.split_at = take(st.gather && st.width == 64 ? 4 * elems : 0);
     const Buf& src = bufs[at[i][0]];
     const Buf& dst = bufs[at[i][2]];
     const int64_t* w = s->ops[i].w;
