@@ -205,25 +205,29 @@ class _UploadSlice:
         return self.up.ready()[self.lo:self.hi]
 
 
+_UPLOAD_LOCK = threading.Lock()
+
+
 def upload_together(tables, recorded: bool = False) -> Uploaded | None:
     """One upload (one staging copy, one device buffer, one event) for the arrays that every
     table in ``tables`` will read and that are not yet on the device, instead of one each
     at its first run.  ``recorded``: the tables are about to be recorded into a sequence.
     Returns the upload, None when there was nothing to do."""
-    todo, arrays = [], []
-    for t in tables:
-        if t is None:
-            continue
-        attr, arrs = t.pending_upload(recorded)
-        if attr is None:
-            continue
-        todo.append((t, attr, len(arrays), len(arrays) + len(arrs)))
-        arrays.extend(arrs)
-    if not todo:
-        return None
-    up = Uploaded(arrays)
-    for t, attr, lo, hi in todo:
-        setattr(t, attr, _UploadSlice(up, lo, hi))
+    with _UPLOAD_LOCK:  # recorded addresses must stay those of the upload a table holds
+        todo, arrays = [], []
+        for t in tables:
+            if t is None:
+                continue
+            attr, arrs = t.pending_upload(recorded)
+            if attr is None:
+                continue
+            todo.append((t, attr, len(arrays), len(arrays) + len(arrs)))
+            arrays.extend(arrs)
+        if not todo:
+            return None
+        up = Uploaded(arrays)
+        for t, attr, lo, hi in todo:
+            setattr(t, attr, _UploadSlice(up, lo, hi))
     return up
 
 
@@ -507,13 +511,16 @@ class GatherTable:
         else:
             items = not CHAIN_DIRECT_GATHER and self.takes_items(True)
         if items:
-            if self._head is None:  # the table's share of the call's arguments
-                rows, tsrc, tcf, tld = self.item_arrays()
-                self._head = (ptr(rows), *self._items[:2], ptr(tsrc), ptr(tcf), ptr(tld),
-                              self.n_term)
+            head = self._head  # (upload, the table's share of the call's arguments from it)
+            if head is None or head[0] is not self._idev:
+                self.item_arrays()
+                up = self._idev
+                rows, tsrc, tcf, tld = up.ready()
+                head = self._head = (up, (ptr(rows), *self._items[:2], ptr(tsrc), ptr(tcf),
+                                          ptr(tld), self.n_term))
             else:
-                self._idev.ready()  # (a run on another stream than the upload's)
-            args = (*self._head, ptr(src0), src0.numel(), ptr(dst0), dst0.numel(),
+                head[0].ready()  # (a run on another stream than the upload's)
+            args = (*head[1], ptr(src0), src0.numel(), ptr(dst0), dst0.numel(),
                     ptr(src1), 0 if src1 is None else src1.numel(),
                     ptr(dst1), 0 if dst1 is None else dst1.numel())
             if rec is not None:

@@ -179,3 +179,21 @@ def test_item_kernel_skips_and_reports_out_of_range_segments():
         assert _lib.device_error(0) != 0
         assert (dst[:600] == 7.0).all()
     assert _lib.device_error(0) == 0
+
+
+@pytest.mark.gpu
+def test_a_second_upload_of_a_table_is_the_one_read():
+    """Two threads that meet at a table's first run may both upload it; a run reads the upload
+    the table holds, never the addresses of one that went away."""
+    import torch
+
+    rng = np.random.default_rng(9)
+    t, n_src, n_dst = _table(rng, [((24, 25), 1), ((6, 7), 3)])
+    src = torch.randn(n_src[0], dtype=torch.float64, device="cuda")
+    want, got = (torch.zeros(n_dst[0], dtype=torch.float64, device="cuda") for _ in range(2))
+    t.run(src, want)
+    first = t._idev
+    t._idev = None
+    t.run(src, got)
+    assert t._idev is not first and t._head[0] is t._idev
+    assert torch.equal(got, want)
