@@ -241,6 +241,9 @@ lanczos_step_kernel(int64_t n, double* w, const double* v, const double* vprev, 
 // of w and v in shared memory, both sums are reduced through distributed shared memory, and
 // two cluster barriers stand where five launches did.  At 68,000 doubles those five launches
 // took about 19 us of kernels and the gaps between them: a 20-step solve 1425 us, now 1078.
+// A peer's shared memory may be written only once that CTA runs, which being scheduled together
+// does not say: every thread arrives at a cluster barrier on entry and waits for it before the
+// first remote store, behind the table search and the loads.
 constexpr int kStepThreads = 512, kStepCluster = 16;
 constexpr int64_t kStepChunk = 8192;  // doubles of w, and of v, per CTA
 
@@ -256,6 +259,7 @@ lanczos_step_cluster_kernel(int64_t n, const double* __restrict__ w,
   double* const sw = step_smem;
   double* const sv = step_smem + chunk;
   const int tid = threadIdx.x, cl = gridDim.x, rank = blockIdx.x;
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   const int64_t lo = static_cast<int64_t>(rank) * chunk;
   const int64_t hi = lo < n ? min(n, lo + chunk) : lo;
   const int len = static_cast<int>(hi - lo);
@@ -272,6 +276,7 @@ lanczos_step_cluster_kernel(int64_t n, const double* __restrict__ w,
   pdl_wait();  // w is the matvec's output
   if (state[3 * ncv + 1] != 0.0) {  // the recurrence already stopped (the same in every CTA)
     for (int i = tid; i < len; i += kStepThreads) vnext[lo + i] = 0.0;
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     return;
   }
 #pragma unroll 8
@@ -280,6 +285,7 @@ lanczos_step_cluster_kernel(int64_t n, const double* __restrict__ w,
     sv[i] = v[lo + i];
   }
   __syncthreads();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // every CTA has started
   // the weighted sum over this chunk, then over the cluster, in a fixed order
   auto dot = [&](const double* x, const double* y, int slot) {
     double acc = 0.0;
