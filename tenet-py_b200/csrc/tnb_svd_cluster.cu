@@ -396,7 +396,8 @@ block_svd_cluster_kernel(const int64_t* __restrict__ rows, int64_t n_rows,
 #pragma unroll
     for (int e = 0; e < E; ++e) {
       const int q = lane + 32 * e;
-      if (q < r && v > 0.0) wout[p * w_col + q * w_el] = w[e] / v;
+      // (a norm that is NaN leaves its column as it is; a zero one is completed below)
+      if (q < r && v != 0.0) wout[p * w_col + q * w_el] = v > 0.0 ? w[e] / v : w[e];
       if (q < c) vout[p * v_col + q * v_el] = z[e];
     }
   };
