@@ -34,7 +34,7 @@ extern "C" {
 #define TNB_EINVAL 1   /* bad argument (null pointer, negative size, bad table)   */
 #define TNB_ECUDA 2    /* a CUDA runtime call failed                               */
 #define TNB_EBOUNDS 3  /* a kernel saw an out-of-range table entry                 */
-#define TNB_ETIMEOUT 4 /* a kernel gave up a bounded wait (tensor-core completion)  */
+#define TNB_ETIMEOUT 4 /* a kernel gave up a bounded wait                            */
 
 /* Maximum tensor rank a gather segment may carry. */
 #define TNB_MAX_RANK 8
@@ -582,6 +582,15 @@ int tnb_block_svd_cluster(const int64_t* rows, int64_t n_rows, const double* a, 
                           double* u, int64_t n_u, double* s, int64_t n_s, double* vt,
                           int64_t n_vt, int32_t* info, int64_t max_r, int64_t max_c,
                           void* stream);
+/*
+ * The same with the limit, in SM clocks, of each wait for a neighbouring column pair
+ * (tnb_block_svd_cluster: about 2 s; 0: each counts as given up).  Where one gives up, the
+ * sector's info is -TNB_ETIMEOUT, its outputs are undefined and the error word is set.
+ */
+int tnb_block_svd_cluster_bounded(const int64_t* rows, int64_t n_rows, const double* a,
+                                  int64_t n_a, double* u, int64_t n_u, double* s, int64_t n_s,
+                                  double* vt, int64_t n_vt, int32_t* info, int64_t max_r,
+                                  int64_t max_c, int64_t wait_cycles, void* stream);
 
 /*
  * The truncation decision on the device: _spectrum / _admissible / _decide of

@@ -18,7 +18,9 @@
 // with cluster-scope release cost 1,500-1,900 clocks a step.  Buffers alternate between two slots: a neighbour sends its step-s columns only
 // after it has read its own step-s buffers, and this warp writes those buffers again only
 // after receiving them, so two slots suffice.  One cluster barrier per sweep decides
-// convergence.
+// convergence.  A warp whose wait gives up leaves the sweep, sends nothing more and says so at
+// that barrier: the whole cluster then stops and the sector's info word is -TNB_ETIMEOUT.  (Its
+// vote, behind the loads of the received columns, takes 1 % of the launch; before them 5 %.)
 //
 // Measured on B200 (the whole launch, before: block_svd_kernel): ten SU(2) sectors up to 116
 // x 116, 2.35 ms (16.5); two 128 x 128 sectors, 2.69 ms (18.9); sectors up to 49 x 49, 0.68
@@ -42,6 +44,7 @@ constexpr int kScRow = 8;  // m, n, a_off, u_off, s_off, vt_off, (w_off), pad
 constexpr int kScMaxSweeps = 64;
 constexpr double kScTol = 1e-15;  // rotate while |a_i . a_j| > tol * |a_i| |a_j|
 constexpr long long kScWaitCycles = 4000000000LL;  // ~2 s at the boost clock
+constexpr long long kScDrainCycles = 200000;  // ~0.1 ms: copies in flight land in microseconds
 
 __device__ __forceinline__ double sc_warp_sum(double v) {
 #pragma unroll
@@ -82,11 +85,12 @@ __device__ __forceinline__ bool sc_test(uint32_t mbar, uint32_t parity, bool rem
         : "=r"(done) : "r"(mbar), "r"(parity) : "memory");
   return done != 0;
 }
-__device__ __forceinline__ bool sc_wait(uint32_t mbar, uint32_t parity, bool remote) {
+__device__ __forceinline__ bool sc_wait(uint32_t mbar, uint32_t parity, bool remote,
+                                        long long limit) {
   if (sc_test(mbar, parity, remote)) return true;
   const long long t0 = clock64();
   while (!sc_test(mbar, parity, remote))
-    if (clock64() - t0 > kScWaitCycles) return false;
+    if (clock64() - t0 > limit) return false;
   return true;
 }
 
@@ -142,10 +146,12 @@ block_svd_cluster_kernel(const int64_t* __restrict__ rows, int64_t n_rows,
                          const double* __restrict__ a, int64_t n_a, double* __restrict__ u,
                          int64_t n_u, double* __restrict__ s, int64_t n_s,
                          double* __restrict__ vt, int64_t n_vt, int32_t* __restrict__ info,
-                         int64_t smem_doubles, int cl) {
+                         int64_t smem_doubles, int cl, long long wait_cycles) {
   extern __shared__ __align__(16) double sc_buf[];
   __shared__ __align__(8) uint64_t mbar[kScMaxWarps][2];
-  __shared__ int rotated[3];
+  // what a sweep's pairs found (1: a rotation, 2: a wait gave up), three sweeps in turn, and the
+  // same for the hand-over after the last sweep
+  __shared__ unsigned rotated[4];
   __shared__ double sig[kScMaxC];
   __shared__ double red[kScMaxWarps];
   const int rank = static_cast<int>(blockIdx.x) % cl;
@@ -194,7 +200,7 @@ block_svd_cluster_kernel(const int64_t* __restrict__ rows, int64_t n_rows,
                    :: "r"(sc_smem(&mbar[warp][q])), "r"(count) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (tid == 0) rotated[0] = rotated[1] = rotated[2] = 0;
+  if (tid < 4) rotated[tid] = 0;
 
   // where slot A (col 0) and slot B (col 1) of this pair go: pair, then slot of the receiver
   const uint32_t slot_bytes = static_cast<uint32_t>(2 * ld * 8);  // one buffer: both columns
@@ -252,14 +258,12 @@ block_svd_cluster_kernel(const int64_t* __restrict__ rows, int64_t n_rows,
                    : "memory");
   };
   if (active) announce(1);
-  bool dead = false;       // a wait gave up: this warp goes on without waiting
+  bool dead = wait_cycles == 0;  // a wait gave up
   uint32_t t = 0;          // steps done; the buffer in use is t & 1
   auto receive = [&]() {   // step t's columns
     const uint32_t slot = t & 1u;
-    if (!dead && !sc_wait(mb0 + 8u * slot, ((t - 1) >> 1) & 1u, remote_in > 0)) {
+    if (!dead && !sc_wait(mb0 + 8u * slot, ((t - 1) >> 1) & 1u, remote_in > 0, wait_cycles))
       dead = true;
-      atomicCAS(&g_device_error, 0, TNB_ETIMEOUT);
-    }
     const double* p = mine + slot * 2 * ld + 2 * lane;
     auto load = [&](const double* q, int groups, double (&x)[E]) {
 #pragma unroll
@@ -275,7 +279,19 @@ block_svd_cluster_kernel(const int64_t* __restrict__ rows, int64_t n_rows,
     load(p + ld, 2 * ew, wb);
     load(p + 64 * ew, 2 * ev, va);
     load(p + ld + 64 * ew, 2 * ev, vb);
-    announce(slot ^ 1u);
+    dead = __any_sync(0xffffffffu, dead);  // the whole warp's
+    if (!dead) announce(slot ^ 1u);
+  };
+  auto report = [&](int word, bool any) {  // to rank 0's words
+    const unsigned found = (any ? 1u : 0u) | (dead ? 2u : 0u);
+    if (found != 0u && lane == 0)
+      asm volatile("red.shared::cluster.or.b32 [%0], %1;" :: "r"(flag0 + 4u * word), "r"(found)
+                   : "memory");
+  };
+  auto reported = [&](int word) {
+    uint32_t f;
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(f) : "r"(flag0 + 4u * word) : "memory");
+    return f;
   };
   // a column to the next step's slot (t already counts that step)
   auto send = [&](const ScDest& d, const double (&w)[E], const double (&v)[E]) {
@@ -298,13 +314,16 @@ block_svd_cluster_kernel(const int64_t* __restrict__ rows, int64_t n_rows,
   };
 
   int sweep = 0;
-  bool converged = c == 1;
-  for (; sweep < kScMaxSweeps && !converged; ++sweep) {
+  bool converged = c == 1, gave_up = false;
+  for (; sweep < kScMaxSweeps && !converged && !gave_up; ++sweep) {
     bool any = false;
     if (active) {
 #pragma unroll 1
       for (int step = 0; step < n1; ++step) {
-        if (t > 0) receive();
+        if (t > 0) {
+          receive();
+          if (dead) break;
+        }
         const int ia = home(0, step), ib = home(1, step);
         if (ia < c && ib < c) {  // (else one is the padding column)
           double aa = 0.0, bb = 0.0, ga = 0.0;
@@ -345,22 +364,21 @@ block_svd_cluster_kernel(const int64_t* __restrict__ rows, int64_t n_rows,
           if (!db.remote) sc_arrive(db.mbar + 8u * (t & 1u));
         }
       }
-      if (any && lane == 0) {
-        const uint32_t f = flag0 + 4u * (sweep % 3);
-        asm volatile("st.shared::cluster.u32 [%0], %1;" :: "r"(f), "r"(1u) : "memory");
-      }
+      report(sweep % 3, any);
     }
     if (rank == 0 && tid == 0) rotated[(sweep + 1) % 3] = 0;
     sc_cluster_sync();
-    uint32_t f;
-    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(f) : "r"(flag0 + 4u * (sweep % 3))
-                 : "memory");
+    const uint32_t f = reported(sweep % 3);  // (the same in every CTA)
     converged = f == 0;
+    gave_up = (f & 2u) != 0;
   }
 
   // singular values: the column norms, to every CTA of the cluster
   const int ia = active ? home(0, 0) : c, ib = active ? home(1, 0) : c;
-  if (active && t > 0) receive();
+  if (active && t > 0 && !gave_up) {
+    receive();
+    report(3, false);
+  }
   double na = 0.0, nb = 0.0;
 #pragma unroll
   for (int e = 0; e < E; ++e) {
@@ -377,6 +395,17 @@ block_svd_cluster_kernel(const int64_t* __restrict__ rows, int64_t n_rows,
       asm volatile("st.shared::cluster.f64 [%0], %1;" :: "r"(p + 8u * ib), "d"(nb) : "memory");
   }
   sc_cluster_sync();
+  if (gave_up || reported(3) != 0u) {  // (the same in every CTA)
+    const long long t0 = clock64();
+    while (clock64() - t0 < kScDrainCycles) {
+    }
+    if (rank == 0 && tid == 0) {
+      atomicCAS(&g_device_error, 0, TNB_ETIMEOUT);
+      info[b] = -TNB_ETIMEOUT;
+    }
+    sc_cluster_sync();  // no CTA leaves while a peer may still read its shared memory
+    return;
+  }
 
   // outputs in descending order (ties by column index): column j goes to position p(j)
   auto position = [&](int j) {
@@ -536,7 +565,16 @@ extern "C" int tnb_block_svd_cluster(const int64_t* rows, int64_t n_rows, const 
                                      int64_t n_a, double* u, int64_t n_u, double* s, int64_t n_s,
                                      double* vt, int64_t n_vt, int32_t* info, int64_t max_r,
                                      int64_t max_c, void* stream) {
-  TNB_REQUIRE(n_rows >= 0 && n_a >= 0 && n_u >= 0 && n_s >= 0 && n_vt >= 0,
+  return tnb_block_svd_cluster_bounded(rows, n_rows, a, n_a, u, n_u, s, n_s, vt, n_vt, info, max_r,
+                                       max_c, tnb::kScWaitCycles, stream);
+}
+
+extern "C" int tnb_block_svd_cluster_bounded(const int64_t* rows, int64_t n_rows, const double* a,
+                                             int64_t n_a, double* u, int64_t n_u, double* s,
+                                             int64_t n_s, double* vt, int64_t n_vt, int32_t* info,
+                                             int64_t max_r, int64_t max_c, int64_t wait_cycles,
+                                             void* stream) {
+  TNB_REQUIRE(n_rows >= 0 && n_a >= 0 && n_u >= 0 && n_s >= 0 && n_vt >= 0 && wait_cycles >= 0,
               "tnb_block_svd_cluster: negative size");
   tnb::ScShape sh;
   TNB_REQUIRE(tnb::sc_shape(max_r, max_c, &sh),
@@ -553,7 +591,8 @@ extern "C" int tnb_block_svd_cluster(const int64_t* rows, int64_t n_rows, const 
     if (x != cudaSuccess) return x;
     return cudaLaunchKernelEx(&cfg, tnb::block_svd_cluster_kernel<E>, rows, n_rows, a, n_a, u,
                               n_u, s, n_s, vt, n_vt, info,
-                              static_cast<int64_t>(sh.smem / 8), sh.cl);
+                              static_cast<int64_t>(sh.smem / 8), sh.cl,
+                              static_cast<long long>(wait_cycles));
   });
   if (e != cudaSuccess) {
     tnb::set_error(std::string("tnb_block_svd_cluster: ") + cudaGetErrorString(e));

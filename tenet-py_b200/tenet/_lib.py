@@ -90,6 +90,8 @@ SIGNATURES = {
     "tnb_block_svd_cluster_ok": (_i32, [_i64, _i64]),
     "tnb_block_svd_cluster": (_i32, [_vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _vp,
                                      _i64, _i64, _vp]),
+    "tnb_block_svd_cluster_bounded": (_i32, [_vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64,
+                                             _vp, _i64, _i64, _i64, _vp]),
     "tnb_truncate_decide": (_i32, [_vp, _vp, _i64, _vp, _i64, _f64, _i32, _f64, _i32, _vp, _vp,
                                    _vp, _vp, _vp]),
     "tnb_svd_compact": (_i32, [_vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _f64, _vp, _i64,
