@@ -635,7 +635,7 @@ int tnb_block_lq(const int64_t* rows, int64_t n_rows, const double* b, int64_t n
                  double* l, int64_t n_l, double* q, int64_t n_q, double* work, int64_t n_work,
                  int64_t smem_doubles, void* stream);
 /*
- * The same factorisation with a sector's columns dealt to 32 warps that hand the reflectors
+ * The same factorisation with a sector's columns dealt to 16 warps that hand the reflectors
  * on without CTA barriers (rows as above, w_off unused).  Takes sectors with nb <= max_nb <=
  * 512 whose mb*nb + 3 min(mb, nb) doubles fit smem_doubles of shared memory.  Same factors
  * and gauge as tnb_block_lq to rounding.
@@ -643,6 +643,14 @@ int tnb_block_lq(const int64_t* rows, int64_t n_rows, const double* b, int64_t n
 int tnb_block_lq_warp(const int64_t* rows, int64_t n_rows, const double* b, int64_t n_b,
                       double* l, int64_t n_l, double* q, int64_t n_q, int64_t max_nb,
                       int64_t smem_doubles, void* stream);
+/*
+ * The same with the limit, in SM clocks, of each wait for a reflector (tnb_block_lq_warp: about
+ * 2 s; 0: each counts as given up).  Where one gives up, the sector's factors are NaN and the
+ * error word is set.
+ */
+int tnb_block_lq_warp_bounded(const int64_t* rows, int64_t n_rows, const double* b, int64_t n_b,
+                              double* l, int64_t n_l, double* q, int64_t n_q, int64_t max_nb,
+                              int64_t smem_doubles, int64_t wait_cycles, void* stream);
 
 
 /* Library version (major*10000 + minor*100 + patch). */

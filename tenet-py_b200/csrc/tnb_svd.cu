@@ -729,7 +729,8 @@ block_lq_kernel(const int64_t* __restrict__ rows, int64_t n_rows, const double* 
 // forms and publishes the next reflector before it turns to its other columns, so the steps'
 // only chain is: the wait, one column's dot product and update, its norm, the reflector's
 // scalars.  Reflectors stay in W below the diagonal; Q's columns are then formed one per warp
-// in registers (column c needs reflectors c..0 only).
+// in registers (column c needs reflectors c..0 only).  Where a wait gives up, the sector's
+// factors are filled with NaN.
 // What bounded block_lq_kernel: per reflector three CTA-wide barriers, a CTA-wide sum and a
 // round of column updates, from global memory where W and Q together do not fit (197 x 77).
 // Measured: seven sectors up to 77 x 197 in 195 us (688 before).  32 warps: 215, 24: 279 (the
@@ -740,9 +741,9 @@ constexpr int kLqThreads = 512, kLqWarps = kLqThreads / 32, kLqMaxRows = 512;
 constexpr long long kLqWaitCycles = 4000000000LL;  // ~2 s at the boost clock
 
 // Wait until the reflector whose mbarrier this is has been published; false when the wait
-// gives up.  (try_wait suspends the warp: 31 warps polling a counter took the shared-memory
+// gives up.  (try_wait suspends the warp: warps that poll a counter take the shared-memory
 // slots that the working ones need.)
-__device__ __forceinline__ bool lq_wait(const double* mbar) {
+__device__ __forceinline__ bool lq_wait(const double* mbar, long long limit) {
   const uint32_t p = static_cast<uint32_t>(__cvta_generic_to_shared(mbar));
   const long long t0 = clock64();
   while (true) {
@@ -753,7 +754,7 @@ __device__ __forceinline__ bool lq_wait(const double* mbar) {
         "selp.b32 %0, 1, 0, p;\n\t}"
         : "=r"(done) : "r"(p) : "memory");
     if (done) return true;
-    if (clock64() - t0 > kLqWaitCycles) return false;
+    if (clock64() - t0 > limit) return false;
   }
 }
 
@@ -762,8 +763,9 @@ __global__ void __launch_bounds__(kLqThreads)
 block_lq_warp_kernel(const int64_t* __restrict__ rows, int64_t n_rows,
                      const double* __restrict__ b, int64_t n_b, double* __restrict__ lout,
                      int64_t n_l, double* __restrict__ qout, int64_t n_q,
-                     int64_t smem_doubles) {
+                     int64_t smem_doubles, long long wait_cycles) {
   extern __shared__ __align__(16) double qr_smem[];
+  __shared__ int gave_up;
   const int64_t blk = blockIdx.x;
   if (blk >= n_rows) return;
   const int64_t* row = rows + blk * kQrRow;
@@ -783,6 +785,7 @@ block_lq_warp_kernel(const int64_t* __restrict__ rows, int64_t n_rows,
   double* const beta = tau + k;
   double* const mbar = beta + k;  // one mbarrier per reflector
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) gave_up = 0;
   for (int e = tid; e < m * n; e += kLqThreads) W[e] = __ldg(b + b_off + e);
   for (int j = tid; j < k; j += kLqThreads)
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;"
@@ -849,16 +852,14 @@ block_lq_warp_kernel(const int64_t* __restrict__ rows, int64_t n_rows,
       if (i >= j && i < m) w[i] = fma(-d, v[e], x[e]);
     }
   };
-  bool dead = false;
+  int dead = wait_cycles == 0;
   if (warp == 0) reflect(0);
   for (int j = 0; j < k; ++j) {
     int c = warp;
     if (c <= j) c += (j - c + kLqWarps) / kLqWarps * kLqWarps;  // the first own column past j
     if (c >= n) break;  // nothing left to update
-    if (!dead && !lq_wait(mbar + j)) {
-      dead = true;  // go on without waiting: every warp reaches the barrier below
-      atomicCAS(&g_device_error, 0, TNB_ETIMEOUT);
-    }
+    if (dead || !lq_wait(mbar + j, wait_cycles))
+      dead = gave_up = 1;  // go on without waiting: every warp reaches the barrier below
     __syncwarp();
     const double t = tau[j];
     double v[E];
@@ -870,6 +871,13 @@ block_lq_warp_kernel(const int64_t* __restrict__ rows, int64_t n_rows,
     }
   }
   __syncthreads();
+  if (gave_up) {
+    if (tid == 0) atomicCAS(&g_device_error, 0, TNB_ETIMEOUT);
+    const double nan = __longlong_as_double(0x7ff8000000000000LL);
+    for (int e = tid; e < n * k; e += kLqThreads) lout[l_off + e] = nan;
+    for (int e = tid; e < k * m; e += kLqThreads) qout[q_off + e] = nan;
+    return;
+  }
 
   // L = R^T (mb x k): row i is column i of R, R[p][i] for p < i, beta on the diagonal
   for (int i = warp; i < n; i += kLqWarps)
@@ -903,7 +911,8 @@ block_lq_warp_kernel(const int64_t* __restrict__ rows, int64_t n_rows,
 template <int E>
 static cudaError_t launch_lq_warp(unsigned grid, int64_t smem_doubles, cudaStream_t s,
                                   const int64_t* rows, int64_t n_rows, const double* b,
-                                  int64_t n_b, double* l, int64_t n_l, double* q, int64_t n_q) {
+                                  int64_t n_b, double* l, int64_t n_l, double* q, int64_t n_q,
+                                  long long wait_cycles) {
   static PerDeviceOnce opted;
   const cudaError_t e = opted.once([] {
     return cudaFuncSetAttribute(block_lq_warp_kernel<E>,
@@ -912,7 +921,7 @@ static cudaError_t launch_lq_warp(unsigned grid, int64_t smem_doubles, cudaStrea
   });
   if (e != cudaSuccess) return e;
   block_lq_warp_kernel<E><<<grid, kLqThreads, static_cast<size_t>(smem_doubles) * 8, s>>>(
-      rows, n_rows, b, n_b, l, n_l, q, n_q, smem_doubles);
+      rows, n_rows, b, n_b, l, n_l, q, n_q, smem_doubles, wait_cycles);
   return cudaSuccess;
 }
 
@@ -947,7 +956,16 @@ extern "C" int tnb_block_lq(const int64_t* rows, int64_t n_rows, const double* b
 extern "C" int tnb_block_lq_warp(const int64_t* rows, int64_t n_rows, const double* b,
                                  int64_t n_b, double* l, int64_t n_l, double* q, int64_t n_q,
                                  int64_t max_nb, int64_t smem_doubles, void* stream) {
-  TNB_REQUIRE(n_rows >= 0 && n_b >= 0 && n_l >= 0 && n_q >= 0, "tnb_block_lq_warp: negative size");
+  return tnb_block_lq_warp_bounded(rows, n_rows, b, n_b, l, n_l, q, n_q, max_nb, smem_doubles,
+                                   tnb::kLqWaitCycles, stream);
+}
+
+extern "C" int tnb_block_lq_warp_bounded(const int64_t* rows, int64_t n_rows, const double* b,
+                                         int64_t n_b, double* l, int64_t n_l, double* q,
+                                         int64_t n_q, int64_t max_nb, int64_t smem_doubles,
+                                         int64_t wait_cycles, void* stream) {
+  TNB_REQUIRE(n_rows >= 0 && n_b >= 0 && n_l >= 0 && n_q >= 0 && wait_cycles >= 0,
+              "tnb_block_lq_warp: negative size");
   TNB_REQUIRE(smem_doubles >= 0 && smem_doubles <= tnb_block_svd_smem_doubles(),
               "tnb_block_lq_warp: shared-memory request beyond the limit");
   TNB_REQUIRE(max_nb >= 0 && max_nb <= tnb::kLqMaxRows,
@@ -956,18 +974,19 @@ extern "C" int tnb_block_lq_warp(const int64_t* rows, int64_t n_rows, const doub
   TNB_REQUIRE(rows && b && l && q, "tnb_block_lq_warp: null pointer");
   TNB_REQUIRE(n_rows < (1ll << 31), "tnb_block_lq_warp: too many sectors");
   const unsigned grid = static_cast<unsigned>(n_rows);
+  const long long limit = wait_cycles;
   cudaStream_t s = tnb::as_stream(stream);
   cudaError_t e;
   if (max_nb <= 32)
-    e = tnb::launch_lq_warp<1>(grid, smem_doubles, s, rows, n_rows, b, n_b, l, n_l, q, n_q);
+    e = tnb::launch_lq_warp<1>(grid, smem_doubles, s, rows, n_rows, b, n_b, l, n_l, q, n_q, limit);
   else if (max_nb <= 64)
-    e = tnb::launch_lq_warp<2>(grid, smem_doubles, s, rows, n_rows, b, n_b, l, n_l, q, n_q);
+    e = tnb::launch_lq_warp<2>(grid, smem_doubles, s, rows, n_rows, b, n_b, l, n_l, q, n_q, limit);
   else if (max_nb <= 128)
-    e = tnb::launch_lq_warp<4>(grid, smem_doubles, s, rows, n_rows, b, n_b, l, n_l, q, n_q);
+    e = tnb::launch_lq_warp<4>(grid, smem_doubles, s, rows, n_rows, b, n_b, l, n_l, q, n_q, limit);
   else if (max_nb <= 256)
-    e = tnb::launch_lq_warp<8>(grid, smem_doubles, s, rows, n_rows, b, n_b, l, n_l, q, n_q);
+    e = tnb::launch_lq_warp<8>(grid, smem_doubles, s, rows, n_rows, b, n_b, l, n_l, q, n_q, limit);
   else
-    e = tnb::launch_lq_warp<16>(grid, smem_doubles, s, rows, n_rows, b, n_b, l, n_l, q, n_q);
+    e = tnb::launch_lq_warp<16>(grid, smem_doubles, s, rows, n_rows, b, n_b, l, n_l, q, n_q, limit);
   if (e != cudaSuccess) {
     tnb::set_error(std::string("tnb_block_lq_warp: ") + cudaGetErrorString(e));
     return TNB_ECUDA;

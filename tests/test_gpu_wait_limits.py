@@ -69,3 +69,34 @@ def test_svd_truncated_raises(monkeypatch):
     linalg.svd_truncated(t, max_bond=5)
     torch.cuda.synchronize()
     assert _lib.device_error(0) == 0
+
+
+@pytest.mark.parametrize("shapes", [[(2, 2)], [(3, 7), (1, 4), (40, 5)], [(77, 197)], [(6, 1)]])
+def test_lq_fills_a_sector_whose_wait_gave_up_with_nan(shapes):
+    rng = np.random.default_rng(5)
+    mats = [rng.standard_normal(s) for s in shapes]
+    rows, bo, lo, qo = [], 0, 0, 0
+    for mb, nb in shapes:
+        k = min(mb, nb)
+        rows.append((mb, nb, bo, lo, qo, -1, 0, 0))
+        bo, lo, qo = bo + mb * nb, lo + mb * k, qo + k * nb
+    B = torch.tensor(np.concatenate([a.ravel() for a in mats]), device="cuda")
+    L, Q = (torch.zeros(x, dtype=torch.float64, device="cuda") for x in (lo, qo))
+    R = torch.tensor(rows, dtype=torch.int64, device="cuda")
+    args = (P(R), len(rows), P(B), B.numel(), P(L), L.numel(), P(Q), Q.numel(),
+            max(nb for _, nb in shapes), max(mb * nb + 3 * min(mb, nb) for mb, nb in shapes))
+    for limit in (0, None):
+        if limit is None:
+            _lib.call("tnb_block_lq_warp", *args, _exec.stream_ptr())
+        else:
+            _lib.call("tnb_block_lq_warp_bounded", *args, limit, _exec.stream_ptr())
+        torch.cuda.synchronize()
+        assert _lib.device_error(0) == (0 if limit is None else TIMEOUT)
+        for (mb, nb, b, l, q, *_), a in zip(rows, mats):
+            k = min(mb, nb)
+            lf, qf = L[l:l + mb * k].cpu().numpy(), Q[q:q + k * nb].cpu().numpy()
+            if limit is None or mb == 1:  # (one row waits for no reflector)
+                got = lf.reshape(mb, k) @ qf.reshape(k, nb)
+                assert np.abs(got - a).max() <= 1e-13 * np.abs(a).max() * max(mb, nb) ** 0.5
+            else:
+                assert np.isnan(lf).all() and np.isnan(qf).all()
