@@ -208,12 +208,21 @@ class _UploadSlice:
 _UPLOAD_LOCK = threading.Lock()
 
 
+def _hold(table, attr: str, arrays) -> None:
+    """Make ``table``'s upload ``attr`` of ``arrays()``, unless another thread just did: under
+    the lock, because launched and recorded addresses must stay those of the one upload the
+    table holds."""
+    with _UPLOAD_LOCK:
+        if getattr(table, attr) is None:
+            setattr(table, attr, Uploaded(arrays()))
+
+
 def upload_together(tables, recorded: bool = False) -> Uploaded | None:
     """One upload (one staging copy, one device buffer, one event) for the arrays that every
     table in ``tables`` will read and that are not yet on the device, instead of one each
     at its first run.  ``recorded``: the tables are about to be recorded into a sequence.
     Returns the upload, None when there was nothing to do."""
-    with _UPLOAD_LOCK:  # recorded addresses must stay those of the upload a table holds
+    with _UPLOAD_LOCK:  # (as in _hold)
         todo, arrays = [], []
         for t in tables:
             if t is None:
@@ -426,7 +435,7 @@ class GatherTable:
 
     def device_arrays(self):
         if self._dev is None:
-            self._dev = Uploaded(self.host_arrays())
+            _hold(self, "_dev", self.host_arrays)
         return self._dev.ready()
 
     @property
@@ -454,7 +463,7 @@ class GatherTable:
 
     def direct_arrays(self):
         if self._ddev is None:
-            self._ddev = Uploaded((self.chunk_rows(), self.tsrc, self.tcf, self.tld))
+            _hold(self, "_ddev", lambda: (self.chunk_rows(), self.tsrc, self.tcf, self.tld))
         return self._ddev.ready()
 
     def item_rows(self):
@@ -491,12 +500,15 @@ class GatherTable:
         if type(self) is GatherTable and self.takes_items(recorded):
             if self._idev is not None:
                 return None, ()
-            return "_idev", (self.item_rows()[2], self.tsrc, self.tcf, self.tld)
+            return "_idev", self.item_host_arrays()
         return ("_dev", self.host_arrays()) if self._dev is None else (None, ())
+
+    def item_host_arrays(self) -> tuple:
+        return (self.item_rows()[2], self.tsrc, self.tcf, self.tld)
 
     def item_arrays(self):
         if self._idev is None:
-            self._idev = Uploaded((self.item_rows()[2], self.tsrc, self.tcf, self.tld))
+            _hold(self, "_idev", self.item_host_arrays)
         return self._idev.ready()
 
     def run(self, src0, dst0, src1=None, dst1=None) -> None:
@@ -667,7 +679,7 @@ class ProductGather(GatherTable):
 
     def device_arrays(self):
         if self._dev is None:
-            self._dev = Uploaded(self.host_arrays())
+            _hold(self, "_dev", self.host_arrays)
         return self._dev.ready()
 
     def run(self, a, b, dst) -> None:
@@ -817,7 +829,7 @@ class GemmTable:
     def device_tables(self):
         """(table, tile_map) on the current device, uploaded on first use."""
         if self._dev is None:
-            self._dev = Uploaded(self.host_arrays())
+            _hold(self, "_dev", self.host_arrays)
         return self._dev.ready()
 
     def slab_rows(self) -> np.ndarray:
@@ -853,7 +865,7 @@ class GemmTable:
         if (rec is None and DIRECT_GEMM and self.tiles >= DIRECT_MIN_TILES
                 and self.kind in (TILE_64, TILE_32, TILE_SKINNY, TILE_WIDE)):
             if self._rows_dev is None:
-                self._rows_dev = Uploaded((self.tile_rows(),))
+                _hold(self, "_rows_dev", lambda: (self.tile_rows(),))
             (rows,) = self._rows_dev.ready()
             mark = _LOG.begin() if _LOG is not None else None
             _lib.call("tnb_grouped_gemm_f64_rows", ptr(rows), self.tiles, self.kind, ptr(a),
@@ -865,7 +877,8 @@ class GemmTable:
         if rec is None and self.kind in (TILE_TC_TF32, TILE_TC_3XBF16) and self.n_counters \
                 and self.tiles >= DIRECT_MIN_TILES:
             if self._rows_dev is None:
-                self._rows_dev = Uploaded((self.table, self.tile_map, self.slab_rows()))
+                _hold(self, "_rows_dev",
+                      lambda: (self.table, self.tile_map, self.slab_rows()))
             table, tile_map, slabs = self._rows_dev.ready()
             mark = _LOG.begin() if _LOG is not None else None
             _lib.call("tnb_grouped_gemm_tc", ptr(table), self.n_gemm, ptr(tile_map), self.tiles,
@@ -1001,7 +1014,7 @@ class GatherAGemm:
 
     def device_tables(self):
         if self._dev is None:
-            self._dev = Uploaded(self.host_arrays())
+            _hold(self, "_dev", self.host_arrays)
         return self._dev.ready()
 
     def private(self):

@@ -1,0 +1,74 @@
+"""A table's device copy is made once, whoever meets at its first use: addresses launched or
+recorded by one thread must not go away because another made a second copy."""
+
+import threading
+import time
+
+import numpy as np
+import pytest
+
+from tenet import _exec
+
+
+class _SlowUpload:
+    """Stands for ``_exec.Uploaded``: takes long enough for a second thread to arrive."""
+
+    made = 0
+
+    def __init__(self, arrays):
+        self.arrays = tuple(_exec._DevArray(64 * (i + 1), x.size) for i, x in enumerate(arrays))
+        time.sleep(0.02)
+        type(self).made += 1
+
+    def ready(self):
+        return self.arrays
+
+
+def _gather():
+    seg = np.zeros((1, _exec.SEG_W), np.int64)
+    seg[0, :5] = 0, 12, 1, 0, 1
+    seg[0, 8] = 12
+    seg[0, 16] = seg[0, 32] = 1
+    return _exec.make_gather((seg, [0], [1.0], [0]))
+
+
+def _gemm(kind):
+    return _exec.make_gemm([(8, 8, 16, 0, 16, 0, 8, 0, 8)], kind)
+
+
+def _run(table, monkeypatch):
+    """``table.run`` up to the library call, as many tiles as the direct forms want."""
+    table.tiles = _exec.DIRECT_MIN_TILES
+    monkeypatch.setattr(type(table), "work", lambda self: None)
+    x = _exec._DevArray(4096, 1024)
+    return lambda: table.run(x, x, x)
+
+
+@pytest.mark.parametrize("use", ["chunk_map", "chunk_rows", "items", "gemm", "gather_a", "rows",
+                                 "slabs", "together"])
+def test_two_threads_make_one_upload(monkeypatch, use):
+    monkeypatch.setattr(_exec, "Uploaded", _SlowUpload)
+    monkeypatch.setattr(_exec, "stream_ptr", lambda: 0)
+    monkeypatch.setattr(_exec._lib, "call", lambda *a: None)
+    _SlowUpload.made = 0
+    if use in ("chunk_map", "chunk_rows", "items"):
+        t = _gather()
+        call = {"chunk_map": t.device_arrays, "chunk_rows": t.direct_arrays,
+                "items": t.item_arrays}[use]
+    elif use == "together":
+        t = _gather()
+        call = lambda: (_exec.upload_together([t]), t.item_arrays())  # noqa: E731
+    elif use == "gather_a":
+        t = _exec.GatherAGemm((np.zeros(129, np.int32), np.zeros(0, np.int32), np.zeros(0)),
+                              [(8, 8, 16, 0, 16, 0, 8, 0, 8)], 128)
+        call = t.device_tables
+    elif use == "gemm":
+        call = _gemm(_exec.TILE_32).device_tables
+    else:
+        call = _run(_gemm(_exec.TILE_32 if use == "rows" else _exec.TILE_TC_3XBF16), monkeypatch)
+    threads = [threading.Thread(target=call) for _ in range(4)]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    assert _SlowUpload.made == 1
