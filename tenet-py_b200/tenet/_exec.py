@@ -823,7 +823,21 @@ class GemmTable:
     def host_arrays(self) -> tuple:
         return (self.table, self.tile_map)
 
+    def takes_rows(self) -> bool:
+        """Whether a launch reads the table from one row per tile, or on the tensor cores per
+        packed slab (a recording never does)."""
+        if self.tiles < DIRECT_MIN_TILES:
+            return False
+        return self.n_counters > 0 if self.kind in (TILE_TC_TF32, TILE_TC_3XBF16) else DIRECT_GEMM
+
+    def rows_host_arrays(self) -> tuple:
+        if self.kind in (TILE_TC_TF32, TILE_TC_3XBF16):
+            return (self.table, self.tile_map, self.slab_rows())
+        return (self.tile_rows(),)
+
     def pending_upload(self, recorded: bool) -> tuple:
+        if not recorded and self.takes_rows():
+            return ("_rows_dev", self.rows_host_arrays()) if self._rows_dev is None else (None, ())
         return ("_dev", self.host_arrays()) if self._dev is None else (None, ())
 
     def device_tables(self):
@@ -862,30 +876,21 @@ class GemmTable:
             return
         work = self.work()
         rec = recording()
-        if (rec is None and DIRECT_GEMM and self.tiles >= DIRECT_MIN_TILES
-                and self.kind in (TILE_64, TILE_32, TILE_SKINNY, TILE_WIDE)):
+        if rec is None and self.takes_rows():
             if self._rows_dev is None:
-                _hold(self, "_rows_dev", lambda: (self.tile_rows(),))
-            (rows,) = self._rows_dev.ready()
+                _hold(self, "_rows_dev", self.rows_host_arrays)
+            rows = self._rows_dev.ready()
+            args = (ptr(a), a.numel(), ptr(b), b.numel(), ptr(c), c.numel(), ptr(work),
+                    self.work_bytes, self.n_counters, stream_ptr())
             mark = _LOG.begin() if _LOG is not None else None
-            _lib.call("tnb_grouped_gemm_f64_rows", ptr(rows), self.tiles, self.kind, ptr(a),
-                      a.numel(), ptr(b), b.numel(), ptr(c), c.numel(), ptr(work),
-                      self.work_bytes, self.n_counters, stream_ptr())
+            if len(rows) == 1:
+                _lib.call("tnb_grouped_gemm_f64_rows", ptr(rows[0]), self.tiles, self.kind, *args)
+            else:
+                _lib.call("tnb_grouped_gemm_tc", ptr(rows[0]), self.n_gemm, ptr(rows[1]),
+                          self.tiles, ptr(rows[2]), self.kind, *args)
             if _LOG is not None:
-                _LOG.end("grouped_gemm_f64", mark, self.flops)
-            return
-        if rec is None and self.kind in (TILE_TC_TF32, TILE_TC_3XBF16) and self.n_counters \
-                and self.tiles >= DIRECT_MIN_TILES:
-            if self._rows_dev is None:
-                _hold(self, "_rows_dev",
-                      lambda: (self.table, self.tile_map, self.slab_rows()))
-            table, tile_map, slabs = self._rows_dev.ready()
-            mark = _LOG.begin() if _LOG is not None else None
-            _lib.call("tnb_grouped_gemm_tc", ptr(table), self.n_gemm, ptr(tile_map), self.tiles,
-                      ptr(slabs), self.kind, ptr(a), a.numel(), ptr(b), b.numel(), ptr(c),
-                      c.numel(), ptr(work), self.work_bytes, self.n_counters, stream_ptr())
-            if _LOG is not None:
-                _LOG.end("grouped_gemm_tc", mark, self.flops)
+                _LOG.end("grouped_gemm_f64" if len(rows) == 1 else "grouped_gemm_tc", mark,
+                         self.flops)
             return
         table, tile_map = self.device_tables()
         if rec is not None:

@@ -72,3 +72,22 @@ def test_two_threads_make_one_upload(monkeypatch, use):
     for th in threads:
         th.join()
     assert _SlowUpload.made == 1
+
+
+@pytest.mark.parametrize("kind", [_exec.TILE_32, _exec.TILE_64, _exec.TILE_SKINNY,
+                                  _exec.TILE_TC_3XBF16])
+@pytest.mark.parametrize("many", [False, True])
+def test_a_launch_uploads_the_form_it_reads(monkeypatch, kind, many):
+    monkeypatch.setattr(_exec, "Uploaded", _SlowUpload)
+    monkeypatch.setattr(_exec, "stream_ptr", lambda: 0)
+    monkeypatch.setattr(_exec._lib, "call", lambda *a: None)
+    t = _gemm(kind)
+    run = _run(t, monkeypatch)
+    t.tiles = _exec.DIRECT_MIN_TILES - (not many)
+    _SlowUpload.made = 0
+    _exec.upload_together([t])
+    run()
+    run()
+    assert _SlowUpload.made == 1 and _exec.upload_together([t]) is None
+    _exec.upload_together([t], recorded=True)  # a recording reads the tile map whatever the size
+    assert _SlowUpload.made == 1 + many and t._dev is not None
