@@ -240,6 +240,25 @@ def upload_together(tables, recorded: bool = False) -> Uploaded | None:
     return up
 
 
+class Fence:
+    """The current stream's work so far, for other streams to wait for."""
+
+    __slots__ = ("stream", "event")
+
+    def __init__(self) -> None:
+        self.stream = stream_ptr()
+        self.event = torch.cuda.Event()
+        self.event.record()
+
+    def wait(self) -> None:
+        if self.event is not None and stream_ptr() != self.stream \
+                and not torch.cuda.is_current_stream_capturing():
+            if self.event.query():
+                self.event = None
+            else:
+                torch.cuda.current_stream().wait_event(self.event)
+
+
 class Uploaded:
     """Device copies of host arrays, made on the current stream.  A copy from pageable
     host memory may still be in flight when the call returns, so a kernel on another
@@ -489,7 +508,7 @@ class GatherTable:
 
     def takes_items(self, recorded: bool) -> bool:
         """Whether a run (or a recording) of this table goes through its warp items."""
-        if not (DIRECT_GATHER and (CHAIN_ITEMS and not _STANDARD[0] if recorded
+        if not (DIRECT_GATHER and (CHAIN_ITEMS and not standard() if recorded
                                    else self.chunks >= DIRECT_MIN_CHUNKS)):
             return False
         return self.item_rows() is not None
@@ -543,7 +562,7 @@ class GatherTable:
             if _LOG is not None:
                 _LOG.end("block_gather", mark, self.bytes_moved)
             return
-        if rec is not None and CHAIN_DIRECT_GATHER and not _STANDARD[0] and self.direct_ok:
+        if rec is not None and CHAIN_DIRECT_GATHER and not standard() and self.direct_ok:
             crows, tsrc, tcf, tld = self.direct_arrays()
             _lib.call("tnb_seq_add_gather_direct", rec.handle, ptr(crows), self.chunks,
                       ptr(tsrc), ptr(tcf), ptr(tld), self.n_term, ptr(src0), src0.numel(),
@@ -596,17 +615,23 @@ DIRECT_MAX_RANK = 4
 #: cold L2 the larger rows cost more than the saved round trips (headline matvec 22.6-25.4
 #: against 21.7-22.6 us, L2 flushed; equal with a warm L2)
 CHAIN_DIRECT_GATHER = False
-_STANDARD = [0]  # > 0 inside standard_gathers()
+
+
+def standard() -> bool:
+    """Whether this thread is inside ``standard_gathers()``."""
+    return getattr(_TLS, "standard", False)
 
 
 @contextmanager
 def standard_gathers():
     """Record chunk-map gathers only (the one-launch chain kernels take no other form)."""
-    _STANDARD[0] += 1
+    before, _TLS.standard = standard(), True
     try:
         yield
     finally:
-        _STANDARD[0] -= 1
+        _TLS.standard = before
+
+
 #: likewise FP64 grouped GEMMs of at least DIRECT_MIN_TILES tiles from one row per tile
 #: (``tnb_grouped_gemm_f64_rows``): one table load per tile instead of two dependent ones
 DIRECT_GEMM = True

@@ -324,16 +324,18 @@ class ChainProgram:
             self.allocate()
         return self
 
+    def _tables(self) -> list:
+        return [t for lk in self.links
+                for t in ((lk.ga, lk.b_gather) if lk.ga is not None else
+                          (lk.a_gather, lk.b_gather, *lk.gemm.parts))] + [self.out_gather]
+
     def allocate(self) -> None:
         """Allocate every buffer once and pack the fixed operands (needs the device)."""
         dev = _exec.device()
         f64 = dict(dtype=torch.float64, device=dev)
         # every table of the chain in one upload, made on the shared template's tables
         # (programs rebound from one template upload once; private copies share it)
-        _exec.upload_together([t for lk in self.links
-                               for t in ((lk.ga, lk.b_gather) if lk.ga is not None else
-                                         (lk.a_gather, lk.b_gather, *lk.gemm.parts))]
-                              + [self.out_gather], recorded=True)
+        _exec.upload_together(self._tables(), recorded=True)
         for lk in self.links:  # split-K scratch of this program's own
             lk.gemm = lk.gemm.private()
         self.a_bufs = [torch.empty(max(1, 0 if lk.ga is not None else lk.a_size), **f64)
@@ -367,9 +369,12 @@ class ChainProgram:
         """A chunk-map recording of the chain's stages, the form the one-launch kernels
         fuse."""
         if self._std_seq is None:
-            self._std_seq = _exec.Seq()
-            with _exec.standard_gathers(), self._std_seq:
-                self._run_tables(self.x_slot, self.y_slot)
+            seq = _exec.Seq()
+            with _exec.standard_gathers():
+                _exec.upload_together(self._tables(), recorded=True)
+                with seq:
+                    self._run_tables(self.x_slot, self.y_slot)
+            self._std_seq = seq
         return self._std_seq
 
     @property
@@ -378,7 +383,7 @@ class ChainProgram:
         fuse (no tensor-core stage, no product-source gather, at most the kernel's stage
         count); else None."""
         if self._fused is None:
-            self._fused = False
+            fused = False
             if (not self.uses_tensor_cores
                     and not any(lk.deferred or lk.ga is not None for lk in self.links)
                     and 0 < len(self.seq) <= FUSED_MAX_STAGES):
@@ -386,7 +391,8 @@ class ChainProgram:
                 fused = _exec.Seq()
                 _lib.call("tnb_seq_fuse", self._standard().handle, self.x_slot.data_ptr(),
                           self.y_slot.data_ptr(), self.barrier.data_ptr(), fused.handle)
-                self._fused = fused
+                self._fused_made = _exec.Fence()  # its tables' uploads and the barrier's zeros
+            self._fused = fused
         return self._fused or None
 
     @property
@@ -396,7 +402,12 @@ class ChainProgram:
         stage-by-stage sequence."""
         if self.cluster is not None and _exec.CLUSTER:
             return self.cluster
-        return (self.fused if _exec.FUSE else None) or self.seq
+        if not _exec.FUSE or (self._fused is None and torch.cuda.is_current_stream_capturing()):
+            return self.seq  # (a graph under capture has no room for the build: the same bits)
+        if self.fused is None:
+            return self.seq
+        self._fused_made.wait()
+        return self.fused
 
     def refresh(self) -> None:
         """Re-pack the fixed operands (after their values changed, same structures)."""
