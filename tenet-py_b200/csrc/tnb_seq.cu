@@ -7,6 +7,7 @@
 // serves every matvec of a solve without host work per launch.  The Lanczos driver
 // launches a whole solve -- ncv matvecs, the recurrence, optional FP64
 // reorthogonalisation -- from one host call; nothing in it waits on the host.
+#include <cmath>
 #include <cstring>
 #include <new>
 #include <string>
@@ -637,14 +638,19 @@ namespace tnb {
 namespace {
 
 // A matvec small enough for tnb_lanczos_small.cu: gathers from warp items and FP64 GEMMs
-// without split sums, every buffer, row and record in shared memory.  That holds bonds up to
-// some 620 elements a vector; there the one launch still takes 262 us where the launches take
-// 466 (420 elements 189 / 465, 134 elements 111 / 382, 26 elements 95 / 341, SU(2) chain, 20
-// vectors), so the multiply-adds of a stage, at most sqrt(|A| |B| |C|) by Hoelder's
-// inequality, and the mean length of its sums, sqrt(|A| |B| / |C|), which one thread adds
-// alone, are only held near what was measured (65,400 and 103).  Fills `a` and returns the
-// shared memory it takes, 0 if it does not fit.
-constexpr double kSmallWork = 98304;
+// without split sums, every buffer, row and record in shared memory, which ends the bonds of a
+// chain first (SU(2): 617 elements).  One SM then does what the launches spread: a step takes it
+// some 55 ps a multiply-add and 0.65 ns an element of a product, the launches some 8 us and 1.8 us
+// a product.  So the multiply-adds of the products, of each at most sqrt(|A| |B| |C|) by
+// Hoelder's inequality, and twelve for each of their elements are held below kSmallWork and
+// kSmallWorkPerProduct for each of them, and the mean length of a product's sums,
+// sqrt(|A| |B| / |C|), which one thread adds alone, where it was measured.
+// Device time of 20 steps in us, one launch / launches: of 150 dense sequences of one to eight
+// products and up to 2,048 elements it takes 141, at 87 to 452 / 214 to 670, none less than 1.12x;
+// two products of 92,160 multiply-adds and 1,920 elements, which it leaves, 273 / 253, three of
+// 65,536 and 2,048 280 / 260.  SU(2) and U(1) chains of 15 to 617 elements 87 to 218 / 460 to
+// 694.  Fills `a` and returns the shared memory it takes, 0 if it does not fit.
+constexpr double kSmallWork = 131072, kSmallWorkPerProduct = 24576, kSmallElement = 12;
 constexpr double kSmallLength = 192;
 constexpr int64_t kSmallMaxN = 2048;
 
@@ -672,6 +678,7 @@ int64_t plan_small(const tnb_seq* s, const void* x_slot, const void* y_slot, int
   if (ix < 0 || iy < 0) return 0;
   int at[kSmallMaxStages][3];
   int64_t rows_bytes = 0;
+  double work = 0.0;  // over the products
   a->n_stages = static_cast<int>(s->ops.size());
   for (int i = 0; i < a->n_stages; ++i) {
     const tnb_seq::Op& op = s->ops[i];
@@ -699,8 +706,8 @@ int64_t plan_small(const tnb_seq* s, const void* x_slot, const void* y_slot, int
         return 0;
       const double na = static_cast<double>(w[6]), nbb = static_cast<double>(w[8]),
                    nc = static_cast<double>(w[10]);
-      if (w[1] > kSmallMaxRows || w[13] != 0 || na * nbb * nc > kSmallWork * kSmallWork ||
-          na * nbb > kSmallLength * kSmallLength * nc)
+      work += std::sqrt(na * nbb * nc) + kSmallElement * nc - kSmallWorkPerProduct;
+      if (w[1] > kSmallMaxRows || w[13] != 0 || na * nbb > kSmallLength * kSmallLength * nc)
         return 0;
       st.count = static_cast<int>(w[1]);
       st.rows = as_ptr(w[0]);
@@ -715,7 +722,7 @@ int64_t plan_small(const tnb_seq* s, const void* x_slot, const void* y_slot, int
         at[i][1] == at[i][2] || at[i][2] == ix)
       return 0;
   }
-  if (bufs[ix].n != n || bufs[iy].n != n) return 0;
+  if (work > kSmallWork || bufs[ix].n != n || bufs[iy].n != n) return 0;
   // buffers that share memory keep to the launches
   int64_t off = 0;
   for (int i = 0; i < nb; ++i) {
