@@ -92,7 +92,9 @@ __device__ bool item_ok(const SmallStage& st, const int* row) {
   if (rank < 1 || rank > kItemMaxRank || ((row[10] >> 8) & 1) || n <= 0 || n > kItemMax ||
       base < 0 || row[6] < 0 || row[7] < row[6] || row[7] > st.n_term)
     return false;
-  int64_t total = 1, lo = item_i64(row[0], row[1]), hi = lo, rr = 0, cc = 0;
+  // row and column offsets of an item of several terms are kept in 16 bits each
+  int64_t total = 1, lo = item_i64(row[0], row[1]), hi = lo;
+  int64_t r_lo = 0, r_hi = 0, c_lo = 0, c_hi = 0;
   for (int d = 0; d < rank; ++d) {
     if (row[12 + d] <= 0) return false;
     total *= row[12 + d];
@@ -100,11 +102,15 @@ __device__ bool item_ok(const SmallStage& st, const int* row) {
     const int64_t x = static_cast<int64_t>(row[12 + d] - 1) * row[20 + d];
     lo += x < 0 ? x : 0;
     hi += x > 0 ? x : 0;
-    if (row[24 + d] < 0 || row[28 + d] < 0) return false;
-    rr += static_cast<int64_t>(row[12 + d] - 1) * row[24 + d];
-    cc += static_cast<int64_t>(row[12 + d] - 1) * row[28 + d];
+    const int64_t r = static_cast<int64_t>(row[12 + d] - 1) * row[24 + d];
+    const int64_t c = static_cast<int64_t>(row[12 + d] - 1) * row[28 + d];
+    (r < 0 ? r_lo : r_hi) += r;
+    (c < 0 ? c_lo : c_hi) += c;
   }
-  if (base + n > total || lo < 0 || hi >= st.n_dst || rr > 65535 || cc > 65535) return false;
+  if (base + n > total || lo < 0 || hi >= st.n_dst) return false;
+  if (row[7] - row[6] > 1 && (r_lo < INT16_MIN || r_hi > INT16_MAX || c_lo < INT16_MIN ||
+                              c_hi > INT16_MAX))
+    return false;
   for (int i = 0; i < row[7] - row[6]; ++i) {
     int64_t ts;
     double cf;
@@ -245,25 +251,27 @@ lanczos_small_kernel(const __grid_constant__ SmallArgs g) {
       if (st.gather) {
         const int* row = reinterpret_cast<const int*>(small_smem + st.rows_at) + k * st.width;
         SmallMove* const rec = reinterpret_cast<SmallMove*>(small_smem + st.recs_at) + at;
-        ushort2* const split = reinterpret_cast<ushort2*>(small_smem + st.split_at) + at;
+        short2* const split = reinterpret_cast<short2*>(small_smem + st.split_at) + at;
         const int rank = row[10] & 255, terms = row[7] - row[6];
         for (int q = lane; q < row[9]; q += 32) {
-          int rem = row[8] + q, rr = 0, cc = 0, to = row[0];
+          int rem = row[8] + q, to = row[0];
+          int64_t rr = 0, cc = 0;
           for (int d = rank - 1; d >= 0; --d) {
             const int quo = d > 0 ? rem / row[12 + d] : 0;
             const int j = rem - quo * row[12 + d];
-            rr += j * row[24 + d];
-            cc += j * row[28 + d];
+            rr += static_cast<int64_t>(j) * row[24 + d];
+            cc += static_cast<int64_t>(j) * row[28 + d];
             to += j * row[20 + d];
             rem = quo;
           }
           SmallMove m;
           m.dst = static_cast<uint16_t>(st.dst + to);
-          m.src = static_cast<uint16_t>(terms > 0 ? st.src + row[2] + row[11] * rr + cc : st.dst);
+          m.src = static_cast<uint16_t>(
+              terms > 0 ? st.src + item_i64(row[2], row[3]) + row[11] * rr + cc : st.dst);
           m.terms = static_cast<uint16_t>(terms);
           m.item = static_cast<uint16_t>(k);
           rec[q] = m;
-          if (st.width == 64) split[q] = make_ushort2(rr, cc);
+          if (st.width == 64) split[q] = make_short2(static_cast<short>(rr), static_cast<short>(cc));
         }
       } else {
         const int64_t* t = static_cast<const int64_t*>(st.rows) + k * TNB_GEMM_WIDTH;
@@ -309,7 +317,7 @@ lanczos_small_kernel(const __grid_constant__ SmallArgs g) {
           const int* row = reinterpret_cast<const int*>(small_smem + st.rows_at) + m.item * st.width;
           double acc = m.terms > 0 ? fma(__hiloint2double(row[5], row[4]), sm[m.src], 0.0) : 0.0;
           if (m.terms > 1) {
-            const ushort2 at = reinterpret_cast<const ushort2*>(small_smem + st.split_at)[e];
+            const short2 at = reinterpret_cast<const short2*>(small_smem + st.split_at)[e];
 #pragma unroll 2
             for (int i = 1; i < m.terms; ++i) {
               int64_t ts;

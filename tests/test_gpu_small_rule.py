@@ -54,3 +54,49 @@ def test_the_work_of_all_products_counts(stages, m, k, one):
                             device="cuda").cpu().numpy().reshape(k, k)
     scale = np.abs(x * y).sum()
     assert abs(state[0] - (x * y).sum()) <= 1e-13 * scale * (stages * k) ** 0.5
+
+
+def _gather(n, kind):
+    """A gather of ``n`` elements, as a user may record one: backwards through the source, or
+    the sum of two terms over a matrix read from its last row up (``n`` = 6 rows)."""
+    row = np.zeros(_exec.SEG_W, np.int64)
+    if kind == "backwards":
+        row[:5] = 0, n, 1, 0, 1
+        row[8], row[16], row[32] = n, 1, -1
+        return _exec.make_gather(([row], [n - 1], [2.0], [0]))
+    c = n // 6
+    row[:5] = 0, n, 2, 0, 2
+    row[8:10], row[16:18], row[24:26], row[32:34] = (6, c), (c, 1), (-1, 0), (0, 1)
+    return _exec.make_gather(([row], [5 * c, 5 * c], [2.0, -0.5], [c, c]))
+
+
+@pytest.mark.parametrize("kind", ["backwards", "rows up"])
+def test_sources_read_backwards(kind, n=48, ncv=5):
+    f64 = dict(dtype=torch.float64, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(2)
+    x_slot, mid, y_slot = (torch.zeros(n, **f64) for _ in range(3))
+    mat, x = torch.randn(n * n, generator=g, **f64), torch.randn(n, generator=g, **f64)
+    gather, gemm = _gather(n, kind), _exec.make_gemm([(1, n, n, 0, n, 0, n, 0, n)], _exec.TILE_32,
+                                                     split_k=False)
+    assert gather.takes_items(True)
+    one, sink = torch.ones(1, **f64), torch.zeros(1, **f64)
+    extra = _exec.make_gemm([(1, 1, 1, 0, 1, 0, 1, 0, 1)], _exec.TILE_32)
+    start, weight = torch.tensor([0, n], device="cuda"), torch.ones(1, **f64)
+    work = torch.zeros(int(_lib.load().tnb_dot_work_bytes(n)), dtype=torch.uint8, device="cuda")
+    out = []
+    for more in (0, 13):  # one launch, and behind more stages than it takes
+        seq = _exec.Seq()
+        with seq:
+            for _ in range(more):
+                extra.run(one, one, sink)
+            gather.run(x_slot, mid)
+            gemm.run(mid, mat, y_slot)
+        V = torch.zeros((ncv + 1, n), **f64)
+        w, state, scal = (torch.zeros(s, **f64) for s in (n, 3 * ncv + 2, 2))
+        _lib.call("tnb_lanczos_solve", seq.handle, P(x_slot), P(y_slot), n, ncv, 1e-30, 0, P(x),
+                  P(V), n, P(w), P(state), P(scal), None, None, P(start), P(weight), 1, P(work),
+                  None, _exec.stream_ptr())
+        torch.cuda.synchronize()
+        assert _lib.device_error(0) == 0 and bool(mid.any()) == bool(more)
+        out.append((V.cpu().numpy(), state.cpu().numpy()))
+    assert all(np.array_equal(a, b) for a, b in zip(*out)) and out[0][0].any()
