@@ -299,16 +299,29 @@ gemm_f64_skinny_kernel(const GemmArgs g) {
 }
 
 // kSkinnyThreads output columns, C[:, n] = A * B[:, n] for M, K <= 16 (the transpose of the
-// skinny case: a few rows, a long N), two columns per thread for K <= 4, else one after the
-// other; loads of B and stores of C run along N, so both are coalesced, and A is a handful
-// of broadcast loads.  Bound by HBM: the descriptor row is one round of loads and B's columns
-// the next, with nothing staged between them, and 48 registers keep ten CTAs on an SM.  768
-// products of up to 4 x 25,790 x 4 (474 MB) take 94.6 us, 5.0 TB/s; one column per thread, A
-// staged behind two barriers, took 240 (six CTAs per SM: 131).
-constexpr int kWideThreads = kSkinnyThreads / 2;
-
-template <int KM, int NC>
+// skinny case: a few rows, a long N); loads of B and stores of C run along N, so both are
+// coalesced.  Bound by HBM, and in a few waves by the chain of loads and sums of one CTA, so
+// the tile's threads and the form of its sums go by the product:
+//   K <= 4, M <= 4  A from broadcast loads, nothing staged: the
+//            descriptor row is one round of loads and B's columns the next, and two columns a
+//            thread at 48 registers keep ten CTAs on an SM;
+//   K <= 16  A's rows in shared memory, padded with zeros to 4, 8, 12 or 16, one column after
+//            the other;
+//   K > 8 and M > 8  the FP64 tensor cores, eight columns a warp at a time.
+// Each element is one chain of fused multiply-adds over k in all of them: the same bits.
+//
+// Threads per tile of 256 columns (builds of the one kernel): 256 up to four tiles an SM, where
+// all CTAs run at once and one column a thread is the shortest chain; 128, two columns a
+// thread, ten CTAs an SM, beyond; between five and eight tiles an SM with 64 registers instead
+// of 48, since ten CTAs are not to be had there.
+// Device times in us, before (a thread per column, A staged behind two barriers) / now: 2,020
+// tiles M = 4 K = 4 10.3 / 5.7, M = 1 K = 16 8.9 / 7.7, M = 16 K = 16 30.4 / 27; 40 tiles M = 16
+// K = 16 3.5 / 2.7, M = 4 K = 4 1.9 / 1.7; 760 tiles, the worst, M = 8 K = 14 7.3 / 8.6.  (Two
+// passes of one column over K > 4 with A from broadcast loads took 59 us and 14.)  768 products
+// of up to 4 x 25,790 x 4 (474 MB) 94.6 us, 5.0 TB/s (240 before).
+template <int KM, int NT>
 __device__ __forceinline__ void wide_columns(const GemmArgs& g, const GemmRow& r, int64_t n) {
+  constexpr int NC = kSkinnyThreads / NT;
   const int M = static_cast<int>(r.M), K = static_cast<int>(r.K);
   const double* const pb = g.b + r.boff + n;
   double bv[NC][KM];
@@ -316,7 +329,7 @@ __device__ __forceinline__ void wide_columns(const GemmArgs& g, const GemmRow& r
   for (int c = 0; c < NC; ++c)
 #pragma unroll
     for (int k = 0; k < KM; ++k)
-      bv[c][k] = k < K && n + c * kWideThreads < r.N ? __ldg(pb + c * kWideThreads + k * r.ldb)
+      bv[c][k] = k < K && n + c * NT < r.N ? __ldg(pb + c * NT + k * r.ldb)
                                                      : 0.0;
   const double* const pa = g.a + r.aoff;
   double* const pc = g.c + r.coff + n;
@@ -334,12 +347,103 @@ __device__ __forceinline__ void wide_columns(const GemmArgs& g, const GemmRow& r
       }
 #pragma unroll
     for (int c = 0; c < NC; ++c)
-      if (n + c * kWideThreads < r.N) pc[m * r.ldc + c * kWideThreads] = s[c];
+      if (n + c * NT < r.N) pc[m * r.ldc + c * NT] = s[c];
   }
 }
 
-__global__ void __launch_bounds__(kWideThreads, 10)
+template <int KM, int NT>
+__device__ __forceinline__ void wide_staged(const GemmArgs& g, const GemmRow& r, int64_t n0,
+                                            double* sa) {
+  const int M = static_cast<int>(r.M), K = static_cast<int>(r.K);
+  for (int i = threadIdx.x; i < M * KM; i += NT)
+    sa[i] = i % KM < K ? __ldg(g.a + r.aoff + (i / KM) * r.lda + (i % KM)) : 0.0;
+  __syncthreads();
+#pragma unroll 1
+  for (int c = 0; c < kSkinnyThreads / NT; ++c) {
+    const int64_t n = n0 + c * NT;
+    if (n >= r.N) return;
+    const double* pb = g.b + r.boff + n;
+    double bv[KM];
+#pragma unroll
+    for (int k = 0; k < KM; ++k) bv[k] = k < K ? __ldg(pb + k * r.ldb) : 0.0;
+    double* pc = g.c + r.coff + n;
+#pragma unroll 2
+    for (int m = 0; m < M; ++m, pc += r.ldc) {
+      const double2* a = reinterpret_cast<const double2*>(sa + m * KM);
+      double s = 0.0;
+#pragma unroll
+      for (int k = 0; k < KM; k += 2) {
+        const double2 v = a[k / 2];
+        s = fma(v.x, bv[k], s);
+        s = fma(v.y, bv[k + 1], s);
+      }
+      *pc = s;
+    }
+  }
+}
+
+// (m8n8k4: ptxas takes no larger FP64 shape under the 48 registers of the many-wave build)
+__device__ __forceinline__ void mma_f64_k4(double (&c)[2], double a, double b) {
+  asm volatile(
+      "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+      : "+d"(c[0]), "+d"(c[1]) : "d"(a), "d"(b));
+}
+
+template <int NT>
+__device__ __forceinline__ void wide_mma(const GemmArgs& g, const GemmRow& r, int64_t tile0) {
+  constexpr int kCols = kSkinnyThreads / (NT / 32);  // a warp's columns
+  const int M = static_cast<int>(r.M), K = static_cast<int>(r.K);
+  const int lane = threadIdx.x & 31, fr = lane >> 2, fk = lane & 3;
+  const int64_t n = tile0 + (threadIdx.x >> 5) * kCols;
+  const int left = static_cast<int>(min(r.N - n, int64_t(kCols)));  // columns to do
+  if (left <= 0) return;
+  double fa[4][2], fb[4];
+#pragma unroll
+  for (int h = 0; h < 4; ++h)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int row = fr + 8 * e, k = 4 * h + fk;
+      fa[h][e] = row < M && k < K ? __ldg(g.a + r.aoff + row * r.lda + k) : 0.0;
+    }
+  const double* pb = g.b + r.boff + n + fr + fk * r.ldb;
+  auto load = [&](int c) {
+#pragma unroll
+    for (int h = 0; h < 4; ++h)
+      fb[h] = c + fr < left && 4 * h + fk < K ? __ldg(pb + c + 4 * h * r.ldb) : 0.0;
+  };
+  double* const pc = g.c + r.coff + n + 2 * fk + fr * r.ldc;
+  const bool pairs = (reinterpret_cast<uintptr_t>(pc) & 15) == 0 && (r.ldc & 1) == 0;
+  load(0);
+#pragma unroll 1
+  for (int c = 0; c < left; c += 8) {
+    double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}}, now[4];
+#pragma unroll
+    for (int h = 0; h < 4; ++h) now[h] = fb[h];
+    if (c + 8 < left) load(c + 8);
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      mma_f64_k4(acc[0], fa[h][0], now[h]);
+      if (M > 8) mma_f64_k4(acc[1], fa[h][1], now[h]);
+    }
+    const int room = left - c - 2 * fk;  // of this lane's two columns
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (fr + 8 * h >= M) continue;
+      double* const p = pc + c + 8 * h * r.ldc;
+      if (pairs && room >= 2) {
+        *reinterpret_cast<double2*>(p) = make_double2(acc[h][0], acc[h][1]);
+      } else {
+        if (room > 0) p[0] = acc[h][0];
+        if (room > 1) p[1] = acc[h][1];
+      }
+    }
+  }
+}
+
+template <int NT, int kMinBlocks>
+__global__ void __launch_bounds__(NT, kMinBlocks)
 gemm_f64_wide_kernel(const GemmArgs g) {
+  __shared__ __align__(16) double sa[kSkinnyMax * kSkinnyMax];
   const int64_t tile = blockIdx.x;
   GemmRow r;
   if (!load_row(g, tile, r) || !footprint_ok(r, g.n_a, g.n_b, g.n_c) || r.M > kSkinnyMax ||
@@ -348,13 +452,32 @@ gemm_f64_wide_kernel(const GemmArgs g) {
     return;
   }
   pdl_wait();  // B may be the previous kernel's output
-  const int64_t n = (tile - r.tile_begin) * kSkinnyThreads + threadIdx.x;
+  const int64_t n0 = (tile - r.tile_begin) * kSkinnyThreads;
   if (r.K <= 4) {
-    wide_columns<4, 2>(g, r, n);
+    if (r.M <= 4)
+      wide_columns<4, NT>(g, r, n0 + threadIdx.x);
+    else
+      wide_staged<4, NT>(g, r, n0 + threadIdx.x, sa);
+  } else if (r.K <= 8) {
+    wide_staged<8, NT>(g, r, n0 + threadIdx.x, sa);
+  } else if (r.M > 8) {
+    wide_mma<NT>(g, r, n0);
+  } else if (r.K <= 12) {
+    wide_staged<12, NT>(g, r, n0 + threadIdx.x, sa);
   } else {
-#pragma unroll 1
-    for (int c = 0; c < 2; ++c) wide_columns<kSkinnyMax, 1>(g, r, n + c * kWideThreads);
+    wide_staged<kSkinnyMax, NT>(g, r, n0 + threadIdx.x, sa);
   }
+}
+
+int device_sms();
+
+static cudaError_t launch_wide(unsigned grid, cudaStream_t s, const GemmArgs& g) {
+  const unsigned sms = static_cast<unsigned>(device_sms());
+  if (grid <= 4 * sms)
+    return launch(gemm_f64_wide_kernel<kSkinnyThreads, 4>, grid, kSkinnyThreads, s, g);
+  if (grid > 5 * sms && grid <= 8 * sms)
+    return launch(gemm_f64_wide_kernel<kSkinnyThreads / 2, 8>, grid, kSkinnyThreads / 2, s, g);
+  return launch(gemm_f64_wide_kernel<kSkinnyThreads / 2, 10>, grid, kSkinnyThreads / 2, s, g);
 }
 
 }  // namespace tnb
@@ -398,7 +521,7 @@ extern "C" int tnb_grouped_gemm_f64(const int64_t* gemm_table, int64_t n_gemm,
       e = tnb::launch(tnb::gemm_f64_skinny_kernel, grid, tnb::kSkinnyThreads, s, g);
       break;
     case TNB_TILE_WIDE:
-      e = tnb::launch(tnb::gemm_f64_wide_kernel, grid, tnb::kWideThreads, s, g);
+      e = tnb::launch_wide(grid, s, g);
       break;
     case TNB_TILE_TC_TF32:
     case TNB_TILE_TC_3XBF16:
@@ -452,7 +575,7 @@ extern "C" int tnb_grouped_gemm_f64_rows(const int64_t* tile_rows, int64_t total
       e = tnb::launch(tnb::gemm_f64_skinny_kernel, grid, tnb::kSkinnyThreads, s, g);
       break;
     default:
-      e = tnb::launch(tnb::gemm_f64_wide_kernel, grid, tnb::kWideThreads, s, g);
+      e = tnb::launch_wide(grid, s, g);
       break;
   }
   if (e != cudaSuccess) {
