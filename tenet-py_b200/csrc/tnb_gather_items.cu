@@ -4,8 +4,9 @@
 // block, write once), the table cut into items of at most 256 consecutive elements of one
 // segment, each one 128- or 256-byte row that a warp reads in one round of loads: offsets,
 // the first terms inline, 32-bit extents, strides and division constants.  A warp moves its
-// item alone: no barrier, no shared memory, all of its loads in flight before the first
-// store.
+// item alone, all loads of a one-term item in flight before the first store; an item of several
+// terms decodes them into the warp's own shared memory.  Large tables of one term a segment and
+// of several have a build each.
 //
 // What bounds it: a many-wave gather (the batched U(1) x U(1) x fZ2 update moves 0.13-0.53 GB
 // a launch in segments of about 600 elements) wants some 45 KB in flight per SM to cover
@@ -26,27 +27,44 @@ namespace tnb {
 
 int device_sms();
 
-// P consecutive items per warp, their rows in flight together.
-template <int NT, int P, int kMinBlocks, bool kRelease>
+template <int NT, int kMinBlocks, bool kRelease, bool kSeveral>
 __global__ void __launch_bounds__(NT, kMinBlocks) gather_items_kernel(const ItemArgs g) {
-  const int lane = threadIdx.x & 31;
-  const int64_t first =
-      (static_cast<int64_t>(blockIdx.x) * (NT / 32) + (threadIdx.x >> 5)) * P;
-  ItemWords w[P];
-#pragma unroll
-  for (int i = 0; i < P; ++i) {
-    if (first + i < g.n_items) {
-      const int32_t* r = g.rows + (first + i) * g.width;
-      w[i].w0 = __ldg(r + lane);
-      w[i].w1 = g.width == 64 ? __ldg(r + 32 + lane) : 0;
-    }
+  __shared__ ItemTerms terms[kSeveral ? NT / 32 : 1];  // (one-term items leave theirs unused)
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t item = static_cast<int64_t>(blockIdx.x) * (NT / 32) + warp;
+  ItemWords w{0, 0};
+  if (item < g.n_items) {
+    const int32_t* r = g.rows + item * g.width;
+    w.w0 = __ldg(r + lane);
+    if (kSeveral && g.width == 64) w.w1 = __ldg(r + 32 + lane);
   }
   pdl_wait<kRelease>();  // the rows are static; the source may be the previous kernel's output
-#pragma unroll
-  for (int i = 0; i < P; ++i) {
-    if (first + i >= g.n_items) return;
-    gather_item_any(g, w[i], lane, [](const double* p) { return __ldg(p); });
-  }
+  if (item < g.n_items)
+    gather_item_any<kSeveral>(g, w, lane, terms[kSeveral ? warp : 0],
+                              [](const double* p) { return __ldg(p); });
+}
+
+// Items of several terms have more registers and fewer warps an SM: under the 64 of 32 warps they
+// spill (3,240 elements of three terms 2.9 us, 2.3 so; 1.9 M of six 48, 40).  Small tables of
+// either kind run the one build: a chain that alternates between two fetches its instructions
+// anew at every launch (a matvec on the L = 64 mid bond 19.4 us, 18.1 so).
+// A warp per item: two items a warp, their rows in flight together, spilled (1.9 M elements in
+// 400 segments 11.2 us, one item 8.6; the batched update the same).  The next kernel is
+// released early only by tables of up to eight warps an SM: from more, its CTAs start while most
+// of this one's data is still to move and hold the SMs meanwhile (3,029 items, a grouped GEMM
+// and 1,515 items of the 40-state U(1) contraction: 52 us released early, 37 not; a compiled
+// matvec on the L = 64 mid bond, 14 to 75 items, gains 2 us a launch from the early release).
+template <bool kSeveral>
+static cudaError_t launch_items(const ItemArgs& g, cudaStream_t s) {
+  const int64_t sms = device_sms(), n = g.n_items;
+  if (n > 32 * sms)
+    return launch(gather_items_kernel<256, kSeveral ? 3 : 4, false, kSeveral>,
+                  static_cast<unsigned>((n + 7) / 8), 256, s, g);
+  if (n > 8 * sms)
+    return launch(gather_items_kernel<128, kSeveral ? 5 : 8, false, kSeveral>,
+                  static_cast<unsigned>((n + 3) / 4), 128, s, g);
+  return launch(gather_items_kernel<128, 5, true, true>,
+                static_cast<unsigned>((n + 3) / 4), 128, s, g);
 }
 
 }  // namespace tnb
@@ -67,24 +85,9 @@ extern "C" int tnb_block_gather_items(const int32_t* item_rows, int32_t width, i
   TNB_REQUIRE(n_items < (int64_t(1) << 31), "tnb_block_gather_items: too many items for one launch");
   const tnb::ItemArgs g{item_rows, width, n_items, term_src, term_coeff, term_ld, n_term,
                         src0, n_src0, dst0, n_dst0, src1, n_src1, dst1, n_dst1};
-  // Beyond one full wave of warps each takes two items, their rows in flight together.  The
-  // next kernel is released early only by tables of up to eight warps an SM: from more, its
-  // CTAs start while most of this one's data is still to move and hold the SMs meanwhile
-  // (3,029 items, a grouped GEMM and 1,515 items of the 40-state U(1) contraction: 52 us
-  // released early, 37 not; a compiled matvec on the L = 64 mid bond, 14 to 75 items, gains
-  // 2 us a launch from the early release).
-  const int64_t sms = tnb::device_sms();
-  cudaStream_t s = tnb::as_stream(stream);
-  cudaError_t e;
-  if (n_items > 32 * sms)
-    e = tnb::launch(tnb::gather_items_kernel<256, 2, 4, false>,
-                    static_cast<unsigned>((n_items + 15) / 16), 256, s, g);
-  else if (n_items > 8 * sms)
-    e = tnb::launch(tnb::gather_items_kernel<128, 1, 8, false>,
-                    static_cast<unsigned>((n_items + 3) / 4), 128, s, g);
-  else
-    e = tnb::launch(tnb::gather_items_kernel<128, 1, 8, true>,
-                    static_cast<unsigned>((n_items + 3) / 4), 128, s, g);
+  const bool several = width == 64 || n_items <= 8 * static_cast<int64_t>(tnb::device_sms());
+  const cudaError_t e = several ? tnb::launch_items<true>(g, tnb::as_stream(stream))
+                                : tnb::launch_items<false>(g, tnb::as_stream(stream));
   if (e != cudaSuccess) {
     tnb::set_error(std::string("tnb_block_gather_items: ") + cudaGetErrorString(e));
     return TNB_ECUDA;

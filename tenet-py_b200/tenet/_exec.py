@@ -444,6 +444,11 @@ class GatherTable:
         self._choice = self._head = None
 
     @property
+    def mean_terms(self) -> float:
+        """Terms per destination element."""
+        return self.term_elems / max(1, self.elems)
+
+    @property
     def bytes_moved(self) -> int:
         """Algorithmic HBM bytes of one run: every term's source read once, every
         destination element written once."""
@@ -492,7 +497,7 @@ class GatherTable:
         if self._items is None:
             lib, seg = _lib.load(), np.ascontiguousarray(self.seg, dtype=np.int64)
             width = 64 if self.n_seg and int((seg[:, 4] - seg[:, 3]).max()) > 1 else 32
-            cap = item_size(self.elems)
+            cap = item_size(self.elems, self.mean_terms)
             args = (self.n_seg, seg.ctypes.data, self.tsrc.ctypes.data, self.tcf.ctypes.data,
                     self.tld.ctypes.data, self.n_term, cap, width)
             n = int(lib.tnb_plan_gather_items(*args, None, 0))
@@ -510,6 +515,8 @@ class GatherTable:
         """Whether a run (or a recording) of this table goes through its warp items."""
         if not (DIRECT_GATHER and (CHAIN_ITEMS and not standard() if recorded
                                    else self.chunks >= DIRECT_MIN_CHUNKS)):
+            return False
+        if self.chunks > ITEM_MANY_CHUNKS and self.mean_terms >= ITEM_MANY_TERMS:
             return False
         return self.item_rows() is not None
 
@@ -604,6 +611,11 @@ class GatherTable:
 #: 1446 us in all), a 974-element one 1.3 against 1.8 us
 DIRECT_GATHER = True
 DIRECT_MIN_CHUNKS = 0
+#: the chunk forms keep tables past ITEM_MANY_CHUNKS chunks with ITEM_MANY_TERMS terms an
+#: element or more: a CTA of theirs reads one term of 1,024 elements after the other, and the
+#: L1 holds the sectors that strided elements share (1.3 M elements of 40 terms 144 us
+#: against 240, 1.9 M of 14 88 against 119; with 6 terms items take 0.6x to 1.16x)
+ITEM_MANY_CHUNKS, ITEM_MANY_TERMS = 2 * 3 * N_SM, 10
 #: record the gathers of compiled chains as warp items too (a matvec on 256 multiplets 36.7
 #: against 39.0 us, with a cold L2 41.0 against 45.0; on the L = 64 mid bond 14.4-16.4 against
 #: 16.4, cold 20.4 against 22.4)
@@ -656,14 +668,18 @@ def chunk_size(sizes, ctas_per_sm: int = GATHER_CTAS_PER_SM) -> int:
     return CHUNK // 4
 
 
-def item_size(elems: int) -> int:
-    """Elements per warp item of a gather of ``elems`` elements: 256, or 128 and 64 for
-    tables that would otherwise leave SMs without a warp.  Smaller items measured slower:
-    more CTAs start for the same bytes (a compiled matvec on 256 multiplets, whose larger
-    gather has 240,000 elements: 36.7 us with 256, 38.4 with 128, 43.7 with 64; at 974 and
-    4,140 elements 64 and 32 are equal)."""
+def item_size(elems: int, terms: float = 1.0) -> int:
+    """Elements per warp item of a gather of ``elems`` elements with ``terms`` terms each on
+    average: 256, or 128 and 64 for tables that would otherwise leave SMs without a warp.
+    With one term a lane has its eight loads in flight at once and smaller items only add
+    CTAs (974 and 4,140 elements: 64 and 32 are equal).  With several a warp walks its terms one
+    round of loads after the other and eight warps an SM take less time (16 for long sums, down
+    to 32 elements): 20 steps of the 256-multiplet solve 1,041 us against 1,091 with one warp
+    an SM, 48,000 elements of 14 terms 5.6 against 9.4."""
+    long = terms >= 8
+    fewest, warps = (32 if long else 64), (1 if terms <= 1 else 16 if long else 8)
     size = 256
-    while size > 64 and elems < size * N_SM:
+    while size > fewest and elems < size * N_SM * warps:
         size //= 2
     return size
 
