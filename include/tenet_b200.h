@@ -578,6 +578,8 @@ int tnb_block_svd(const int64_t* rows, int64_t n_rows, const double* a, int64_t 
  * as tnb_block_svd to rounding, in the same gauge.
  */
 int tnb_block_svd_cluster_ok(int64_t max_r, int64_t max_c);
+/* How many sectors of a launch with these bounds run at the same time (0: not taken). */
+int64_t tnb_block_svd_cluster_count(int64_t max_r, int64_t max_c);
 int tnb_block_svd_cluster(const int64_t* rows, int64_t n_rows, const double* a, int64_t n_a,
                           double* u, int64_t n_u, double* s, int64_t n_s, double* vt,
                           int64_t n_vt, int32_t* info, int64_t max_r, int64_t max_c,

@@ -544,9 +544,13 @@ static auto sc_dispatch(int64_t r, F&& f) {
 }  // namespace tnb
 
 extern "C" int tnb_block_svd_cluster_ok(int64_t max_r, int64_t max_c) {
+  return tnb_block_svd_cluster_count(max_r, max_c) > 0 ? 1 : 0;
+}
+
+extern "C" int64_t tnb_block_svd_cluster_count(int64_t max_r, int64_t max_c) {
   tnb::ScShape sh;
   if (!tnb::sc_shape(max_r, max_c, &sh)) return 0;
-  const int clusters = tnb::sc_dispatch(max_r, [&](auto tag) {
+  return tnb::sc_dispatch(max_r, [&](auto tag) {
     constexpr int E = decltype(tag)::value;
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[1];
@@ -558,7 +562,6 @@ extern "C" int tnb_block_svd_cluster_ok(int64_t max_r, int64_t max_c) {
     }
     return n;
   });
-  return clusters > 0 ? 1 : 0;
 }
 
 extern "C" int tnb_block_svd_cluster(const int64_t* rows, int64_t n_rows, const double* a,

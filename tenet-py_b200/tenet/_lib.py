@@ -88,6 +88,7 @@ SIGNATURES = {
     "tnb_block_svd": (_i32, [_vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64,
                              _vp, _i64, _vp]),
     "tnb_block_svd_cluster_ok": (_i32, [_i64, _i64]),
+    "tnb_block_svd_cluster_count": (_i64, [_i64, _i64]),
     "tnb_block_svd_cluster": (_i32, [_vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _vp,
                                      _i64, _i64, _vp]),
     "tnb_block_svd_cluster_bounded": (_i32, [_vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64,

@@ -103,6 +103,60 @@ def _raise_exec(s: TensorStructure):
                                                terms))
 
 
+def _svd_doubles(r: int, c: int) -> int:
+    """Working copy of an r x c sector (r >= c) in ``tnb_block_svd``."""
+    return r * c + c * c + 2 * c
+
+
+#: the largest sector ``tnb_block_svd_cluster`` takes
+CLUSTER_ROWS, CLUSTER_COLS = 512, 256
+
+
+def cluster_sectors(shapes: dict, count, smem_doubles: int) -> dict:
+    """Which sectors ``{label: (rows, columns)}`` (rows >= columns) go to
+    ``tnb_block_svd_cluster``, the others to ``tnb_block_svd``: the same bits, so only time
+    decides.  ``count(rows, columns)``: sectors of a launch that run at once, 0 when it cannot.
+
+    The cluster hands every column on after each step, which pays where one CTA would need
+    several rounds a step (over 32 columns: 0.2x to 0.65x of its time) and for most smaller
+    ones (down to 0.6x), but not
+    - for long thin sectors (32 columns or less in shared memory, and over 256 rows or at least
+      32 rows a column): 1.05x to 1.9x (512 x 10 160 us against 91).  They change over where no
+      other sector is left in the launch, or where its columns get shorter by it;
+    - past the clusters that run at once: 148 sectors of 192 x 20 1.7x, of 96 x 32 1.3x;
+    - beside a larger sector past both its limits and one CTA's shared memory, for sectors that
+      work in global memory there too: 256 x 256 and 300 x 300 153 ms in two launches, 148 in
+      one.  (Those that would take shared memory take the larger one's L1: 64 x 64 and 300 x 300
+      147 ms in two launches, 159 in one.)"""
+    fit = {k: x for k, x in shapes.items() if x[0] <= CLUSTER_ROWS and x[1] <= CLUSTER_COLS}
+    cost = lambda x: x[0] * x[1] * x[1]  # noqa: E731
+    small = lambda x: _svd_doubles(*x) <= smem_doubles  # noqa: E731
+    large = max((cost(x) for k, x in shapes.items() if k not in fit and not small(x)), default=0)
+    if large and len(shapes) <= _exec.N_SM:
+        fit = {k: x for k, x in fit.items() if small(x) or cost(x) > large}
+
+    def thin(x) -> bool:
+        r, c = x
+        return not large and c <= 32 and small(x) and (r > 256 or 32 * c <= r)
+
+    rest = {k: x for k, x in fit.items() if not thin(x)}
+    if not rest:
+        return {}
+    if not large and max(r for r, _ in rest.values()) <= 256:
+        fit = {k: x for k, x in fit.items() if x[0] <= 256}
+    r, c = max(x[0] for x in fit.values()), max(x[1] for x in fit.values())
+    at_once = count(r, c)
+    if not at_once:
+        return {}
+    waves = -(-len(fit) // at_once)
+    need = max(_svd_doubles(*x) for x in fit.values())
+    if waves > 1 and need <= smem_doubles and not large:
+        per_sm = min(4, smem_doubles // need)  # (512 threads a CTA)
+        if (0.8 if c <= 32 else 0.35) * waves >= -(-len(fit) // (_exec.N_SM * per_sm)):
+            return {}
+    return fit
+
+
 class _SvdPlan:
     """Device tables of one lowered structure's blockwise SVD: per coupled sector (in label
     order) its shape and the offsets of its full factors, the decision's sector table,
@@ -121,15 +175,12 @@ class _SvdPlan:
         self.kfull = {}
         uo = so = vo = wo = 0
         smem = 0
-        # the sectors a cluster launch takes come first: all but the largest ones
-        shapes = sorted((max(ml.shape[c]), min(ml.shape[c]), c) for c in self.sectors)
-        while shapes and not lib.tnb_block_svd_cluster_ok(
-                max(x[0] for x in shapes), max(x[1] for x in shapes)):
-            shapes.pop()
-        clustered = {c for _, _, c in shapes}
-        self.n_cluster = len(shapes)
-        self.max_r = max((x[0] for x in shapes), default=0)
-        self.max_c = max((x[1] for x in shapes), default=0)
+        # the sectors of the cluster launch come first
+        clustered = cluster_sectors({c: (max(ml.shape[c]), min(ml.shape[c])) for c in self.sectors},
+                                    lib.tnb_block_svd_cluster_count, smem_max)
+        self.n_cluster = len(clustered)
+        self.max_r = max((r for r, _ in clustered.values()), default=0)
+        self.max_c = max((c for _, c in clustered.values()), default=0)
         for c in self.sectors:
             r, q = ml.shape[c]
             k = min(r, q)
