@@ -818,9 +818,13 @@ extern "C" int tnb_lanczos_solve(const tnb_seq* matvec, const void* x_slot, cons
   TNB_TRY(tnb_scale_rsqrt(n, scal, x0, v, stream));
   const void* from[2] = {x_slot, y_slot};
   // a vector one CTA can carry takes each step's five vector launches as one
-  // (up to 8,192 doubles), or one cluster of CTAs (up to 131,072)
+  // (up to 8,192 doubles), or one cluster of CTAs (up to 131,072).  Its 16 CTAs walk the runs of
+  // equal weights one after the other where the launches' sums have a CTA for every few: with
+  // 2,000 runs 20 steps take 1,456 us of 68,000 doubles (launches 1,793), but 1,480 of 131,072
+  // (1,341).  A solve without runs keeps to the launches, which take it.
   const bool one_cta = !reorth && n <= tnb_lanczos_step_max_n();
-  const bool cluster = !reorth && !one_cta && n <= tnb_lanczos_step_cluster_max_n();
+  const bool cluster = !reorth && !one_cta && n_runs > 0 && (n_runs <= 1024 || n <= 81920) &&
+                       n <= tnb_lanczos_step_cluster_max_n();
   for (int32_t j = 0; j < ncv; ++j) {
     double* vj = v + static_cast<int64_t>(j) * ldv;
     void* to[2] = {vj, w};

@@ -100,3 +100,40 @@ def test_sources_read_backwards(kind, n=48, ncv=5):
         assert _lib.device_error(0) == 0 and bool(mid.any()) == bool(more)
         out.append((V.cpu().numpy(), state.cpu().numpy()))
     assert all(np.array_equal(a, b) for a, b in zip(*out)) and out[0][0].any()
+
+
+@pytest.mark.parametrize("n, runs", [(8193, 0), (100000, 1500), (100000, 3)])
+def test_long_solves_of_any_runs(n, runs, ncv=3):
+    """No runs (every sum is zero), more than the cluster step takes at this length, few."""
+    f64 = dict(dtype=torch.float64, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(n + runs)
+    x_slot, y_slot = (torch.zeros(n, **f64) for _ in range(2))
+    row = np.zeros(_exec.SEG_W, np.int64)
+    row[:5] = 0, n, 1, 0, 1
+    row[8], row[16], row[32] = n, 1, -1
+    gather = _exec.make_gather(([row], [n - 1], [1.5], [0]))  # 1.5 x backwards
+    seq = _exec.Seq()
+    with seq:
+        gather.run(x_slot, y_slot)
+    cuts = np.linspace(0, n, runs + 1).astype(np.int64)
+    wts = np.arange(1.0, runs + 1.0) % 5 + 1
+    start = torch.tensor(cuts, device="cuda")
+    weight = torch.tensor(np.append(wts, 1.0), device="cuda")
+    x = torch.randn(n, generator=g, **f64)
+    V = torch.zeros((ncv + 1, n), **f64)
+    w, state, scal = (torch.zeros(s, **f64) for s in (n, 3 * ncv + 2, 2))
+    work = torch.zeros(int(_lib.load().tnb_dot_work_bytes(n)), dtype=torch.uint8, device="cuda")
+    _lib.call("tnb_lanczos_solve", seq.handle, P(x_slot), P(y_slot), n, ncv, 1e-30, 0, P(x), P(V),
+              n, P(w), P(state), P(scal), None, None, P(start), P(weight), runs, P(work),
+              None, _exec.stream_ptr())
+    torch.cuda.synchronize()
+    assert _lib.device_error(0) == 0
+    if not runs:
+        assert float(scal[0]) == 0.0
+        return
+    q, xh = np.repeat(wts, np.diff(cuts)), x.cpu().numpy()
+    v = xh / np.sqrt(np.sum(q * xh * xh))
+    a = np.sum(q * v * 1.5 * v[::-1])
+    assert abs(float(state[0]) - a) <= 1e-12 * np.sum(q * np.abs(v * v[::-1]))
+    r = 1.5 * v[::-1] - a * v
+    assert abs(float(state[2 * ncv]) - np.sum(q * r * r)) <= 1e-11 * np.sum(q * r * r)
