@@ -140,10 +140,11 @@ CLUSTER_CTAS = 16
 
 
 class _Staging:
-    """A pinned host ring through which plan tables reach the device: a table is packed
-    into the next free bytes of the ring and copied asynchronously, so an upload costs a
-    host memcpy and one queued copy.  Before the ring wraps, every copy still reading it
-    is waited for."""
+    """A pinned host ring through which plan tables reach the device: an upload's arrays are
+    written into the next free bytes of the ring and copied asynchronously, so an upload
+    costs a host memcpy and one queued copy.  Before the ring wraps, every copy still
+    reading it is waited for.  ``lock`` is held from the writing to the copy's event, so that
+    no other thread wraps the ring in between."""
 
     def __init__(self, nbytes: int = 64 << 20) -> None:
         self.nbytes = nbytes
@@ -152,12 +153,9 @@ class _Staging:
         self.pending: list = []
         self.lock = threading.Lock()
 
-    def stage(self, packed: np.ndarray):
-        with self.lock:
-            return self._stage(packed)
-
-    def _stage(self, packed: np.ndarray):
-        n = packed.nbytes
+    def stage(self, arrays, offsets, n: int):
+        """The ring's bytes that hold ``arrays`` at ``offsets`` (``n`` in all), None when they
+        are too many."""
         if n > self.nbytes // 4:
             return None
         if self.buf is None:
@@ -169,7 +167,9 @@ class _Staging:
             self.pending.clear()
             self.pos = 0
         view = self.buf[self.pos:self.pos + n]
-        self.host[self.pos:self.pos + n] = packed
+        host = self.host[self.pos:self.pos + n]
+        for x, o in zip(arrays, offsets):
+            host[o:o + x.nbytes] = x.reshape(-1).view(np.uint8)
         self.pos = -(-(self.pos + n) // 256) * 256
         return view
 
@@ -270,30 +270,33 @@ class Uploaded:
     __slots__ = ("arrays", "stream", "event", "buf")
 
     def __init__(self, host_arrays) -> None:
-        # one host->device copy: the arrays packed at 16-byte aligned offsets of one
-        # buffer, then typed views into its device copy
+        # one host->device copy: the arrays at 16-byte aligned offsets of one buffer, then typed
+        # views into its device copy
         host_arrays = [np.ascontiguousarray(x) for x in host_arrays]
         offs, total = [], 0
         for x in host_arrays:
             offs.append(total)
             total += -(-x.nbytes // 16) * 16
-        packed = np.zeros(max(total, 16), dtype=np.uint8)
-        for x, o in zip(host_arrays, offs):
-            packed[o:o + x.nbytes] = x.reshape(-1).view(np.uint8)
-        staged = None if torch.cuda.is_current_stream_capturing() else _STAGING.stage(packed)
-        if staged is not None:
-            dev_buf = torch.empty(packed.nbytes, dtype=torch.uint8, device=device())
-            dev_buf.copy_(staged, non_blocking=True)
-        else:
-            dev_buf = torch.from_numpy(packed).to(device())
-        base = dev_buf.data_ptr()
-        self.buf = dev_buf
+        total = max(total, 16)
+        self.event = torch.cuda.Event()
+        self.buf = None
+        if not torch.cuda.is_current_stream_capturing():
+            with _STAGING.lock:
+                staged = _STAGING.stage(host_arrays, offs, total)
+                if staged is not None:
+                    self.buf = torch.empty(total, dtype=torch.uint8, device=device())
+                    self.buf.copy_(staged, non_blocking=True)
+                    self.event.record()
+                    _STAGING.pending.append(self.event)
+        if self.buf is None:
+            packed = np.zeros(total, dtype=np.uint8)
+            for x, o in zip(host_arrays, offs):
+                packed[o:o + x.nbytes] = x.reshape(-1).view(np.uint8)
+            self.buf = torch.from_numpy(packed).to(device())
+            self.event.record()
+        base = self.buf.data_ptr()
         self.arrays = tuple(_DevArray(base + o, x.size) for x, o in zip(host_arrays, offs))
         self.stream = stream_ptr()
-        self.event = torch.cuda.Event()
-        self.event.record()
-        if staged is not None:
-            _STAGING.pending.append(self.event)
 
     def ready(self) -> tuple:
         if self.event is not None and stream_ptr() != self.stream \
@@ -500,15 +503,12 @@ class GatherTable:
             cap = item_size(self.elems, self.mean_terms)
             args = (self.n_seg, seg.ctypes.data, self.tsrc.ctypes.data, self.tcf.ctypes.data,
                     self.tld.ctypes.data, self.n_term, cap, width)
-            n = int(lib.tnb_plan_gather_items(*args, None, 0))
+            most = int(((seg[:, 1] + cap - 1) // cap).sum()) if self.n_seg else 0
+            rows = np.empty((most, width), dtype=np.int32)
+            n = int(lib.tnb_plan_gather_items(*args, rows.ctypes.data, most))
             if n < -1:
                 raise ValueError("item_rows: a malformed gather table")
-            self._items = False
-            if n > 0:
-                rows = np.empty((n, width), dtype=np.int32)
-                if int(lib.tnb_plan_gather_items(*args, rows.ctypes.data, n)) != n:
-                    raise ValueError("item_rows: a malformed gather table")
-                self._items = (width, n, rows)
+            self._items = (width, n, rows[:n]) if n > 0 else False
         return self._items or None
 
     def takes_items(self, recorded: bool) -> bool:

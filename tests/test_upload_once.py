@@ -91,3 +91,57 @@ def test_a_launch_uploads_the_form_it_reads(monkeypatch, kind, many):
     assert _SlowUpload.made == 1 and _exec.upload_together([t]) is None
     _exec.upload_together([t], recorded=True)  # a recording reads the tile map whatever the size
     assert _SlowUpload.made == 1 + many and t._dev is not None
+
+
+def test_uploads_never_share_staging_bytes(monkeypatch):
+    """Two threads upload through a ring that wraps at every second upload: the bytes of one are
+    not written over before its copy has been queued."""
+    class Buffer:
+        def __init__(self, n):
+            self.data = np.zeros(n, np.uint8)
+
+        def pin_memory(self):
+            return self
+
+        def numpy(self):
+            return self.data
+
+        def __getitem__(self, part):
+            return self.data[part]
+
+        def copy_(self, staged, non_blocking):
+            time.sleep(0.002)  # (a thread that wraps the ring meanwhile would overwrite it)
+            self.data[:] = staged
+
+        def data_ptr(self):
+            return 64
+
+    class Event:
+        def record(self):
+            pass
+
+        def synchronize(self):
+            pass
+
+    monkeypatch.setattr(_exec.torch, "empty", lambda n, **k: Buffer(n))
+    monkeypatch.setattr(_exec.torch.cuda, "Event", Event)
+    monkeypatch.setattr(_exec.torch.cuda, "is_current_stream_capturing", lambda: False)
+    monkeypatch.setattr(_exec, "device", lambda: None)
+    monkeypatch.setattr(_exec, "stream_ptr", lambda: 0)
+    monkeypatch.setattr(_exec, "_STAGING", _exec._Staging(4096))
+    bad = []
+
+    def upload(value):
+        for k in range(20):
+            x, y = np.full(100, value + k), np.full(3, value - k, np.int32)
+            got = _exec.Uploaded((x, y))
+            if not (np.array_equal(got.buf.data[:800].view(np.int64), x)
+                    and np.array_equal(got.buf.data[800:812].view(np.int32), y)):
+                bad.append((value, k))
+
+    threads = [threading.Thread(target=upload, args=(1000 * t,)) for t in range(4)]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    assert not bad
