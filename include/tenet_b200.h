@@ -115,7 +115,8 @@ int tnb_block_gather_direct(const int64_t* chunk_rows, int64_t total_chunks,
 
 /*
  * The same block maps from warp items: the table as one row of `width` int32 words (32, or
- * 64 with up to six further terms inline) per item, an item being at most
+ * 64 with up to six further terms inline: the form for tables of several terms a segment; rows of
+ * 32 take them too, slowly) per item, an item being at most
  * TNB_ITEM_MAX_ELEMS consecutive elements of a segment (rank <= 4, offsets within a segment
  * below 2^31).  Words: [0,1] destination offset, [2,3] first term's source, [4,5] its
  * coefficient (64-bit values, low word first), [6] first and [7] past-the-last term, [8]
@@ -483,9 +484,10 @@ int tnb_seq_run(const tnb_seq* s, int32_t n_patch, const void* const* from, void
  * optional classical Gram-Schmidt twice against v_0..v_j (reorth != 0; vptrs = DEVICE
  * array of the ncv row pointers of v, gs = ncv doubles, multi_work of
  * tnb_multi_dot_work_bytes(n, ncv) bytes), ||w||^2 and tnb_lanczos_next.  `v` holds
- * ncv + 1 rows of stride ldv >= n; `scal` 2 doubles; dot_work tnb_dot_work_bytes(n).
+ * ncv + 1 rows of stride ldv >= n; `scal` 2 doubles; dot_work tnb_dot_work_bytes(n); `w` is
+ * scratch (what it holds afterwards depends on the form below).
  * Without reorthogonalisation the vector work of a step is one launch up to
- * tnb_lanczos_step_cluster_max_n() doubles, and a matvec of recorded gather items and FP64
+ * tnb_lanczos_step_cluster_max_n() doubles (past 81,920 with at most 1,024 runs), and a matvec of recorded gather items and FP64
  * GEMMs without split sums whose buffers, rows and records fit one SM's shared memory (214
  * KB; some 620 elements of an SU(2) chain) makes the whole solve one launch of one CTA, with
  * the same bits; the recorded buffers between its stages are then read and not written.
@@ -574,8 +576,8 @@ int tnb_block_svd(const int64_t* rows, int64_t n_rows, const double* a, int64_t 
  * The same factorisation with each sector on a thread-block cluster, a warp per column pair
  * (rows as above, w_off unused).  Takes sectors with max(m, n) <= max_r <= 512 and
  * min(m, n) <= max_c <= 256; tnb_block_svd_cluster_ok says whether a launch with these
- * bounds can run on the current device (1) or not (0).  Same singular values and vectors
- * as tnb_block_svd to rounding, in the same gauge.
+ * bounds can run on the current device (1) or not (0).  Same bits as tnb_block_svd (a NaN
+ * norm has no order among several columns in either).
  */
 int tnb_block_svd_cluster_ok(int64_t max_r, int64_t max_c);
 /* How many sectors of a launch with these bounds run at the same time (0: not taken). */

@@ -15,8 +15,10 @@
 // offsets, with every check of the launched stages made there: decoding the items in every step
 // took 2,100 to 9,000 clocks a gather, a solve at 194 elements 305 us.
 //
-// Measured on B200, 20 vectors, from the call to the result: 26 elements 365 -> 111 us, 134
-// elements 399 -> 128, 420 elements 477 -> 203, 617 elements 482 -> 277; a 16-site sweep 28.8 -> 20.8 ms.
+// Measured on B200, 20 vectors, from the call to the result read on the host (device times, and
+// the rule that takes a matvec here: plan_small in tnb_seq.cu): 26 elements 365 -> 111 us, 134
+// elements 399 -> 128, 420 elements 477 -> 203, 617 elements 482 -> 277; a 16-site sweep 28.8 ->
+// 20.8 ms.
 //
 // Same arithmetic as the launches it replaces, in the same order (an element of a product as one
 // chain of fused multiply-adds over k, gathers in table order, the recurrence rounded operation

@@ -15,15 +15,15 @@
 // straight into its neighbours' shared memory and signals the receiver's mbarrier; no step
 // has a barrier.  Within a CTA that is a plain store and an arrive, across CTAs st.async,
 // whose bytes complete the receiver's mbarrier themselves: a store followed by an arrive
-// with cluster-scope release cost 1,500-1,900 clocks a step.  Buffers alternate between two slots: a neighbour sends its step-s columns only
-// after it has read its own step-s buffers, and this warp writes those buffers again only
-// after receiving them, so two slots suffice.  One cluster barrier per sweep decides
+// with cluster-scope release cost 1,500-1,900 clocks a step.  Buffers alternate between two
+// slots: a neighbour sends its step-s columns only after it has read its own step-s buffers, and
+// this warp writes those buffers again only after receiving them, so two slots suffice.  One cluster barrier per sweep decides
 // convergence.  A warp whose wait gives up leaves the sweep, sends nothing more and says so at
 // that barrier: the whole cluster then stops and the sector's info word is -TNB_ETIMEOUT.  (Its
 // vote, behind the loads of the received columns, takes 1 % of the launch; before them 5 %.)
 //
 // Measured on B200 (the whole launch, before: block_svd_kernel): ten SU(2) sectors up to 116
-// x 116, 2.35 ms (16.5); two 128 x 128 sectors, 2.69 ms (18.9); sectors up to 49 x 49, 0.68
+// x 116, 2.4 ms (16.5); two 128 x 128 sectors, 2.7 ms (18.9); sectors up to 49 x 49, 0.68
 // ms (2.18); up to 22 x 22, 0.24 ms (0.34); up to 5 x 5, 30 us (32) -- the same sweeps and the
 // same bits.  A step of 128 columns is about 1,800 clocks: dot products and their shuffles
 // 350, the divide / square root chain 470, rotation and sends 300, and the rest the
@@ -31,7 +31,8 @@
 // slower, 3.2 against 2.35 ms: every mbarrier wait costs some 250 clocks even when it is ready.
 //
 // Limits: max(m, n) <= 512 and min(m, n) <= 256 (the columns of at most eight pairs, two
-// slots each, in one CTA's shared memory); larger sectors take block_svd_kernel.
+// slots each, in one CTA's shared memory); larger sectors, and those it is slower for
+// (linalg.cluster_sectors), take block_svd_kernel.
 #include <string>
 #include <type_traits>
 
