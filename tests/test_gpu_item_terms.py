@@ -53,9 +53,9 @@ def test_many_items(copies):
 
 
 @pytest.mark.parametrize("width", [32, 64])
-@pytest.mark.parametrize("cap", [32, 64, 96, 256])
-def test_rows_of_either_width(width, cap):
-    _run([0, 1, 2, 8, 40], 1, width, cap)
+@pytest.mark.parametrize("cap, copies", [(32, 1), (64, 1), (96, 1), (256, 1), (64, 12), (32, 30)])
+def test_rows_of_either_width(width, cap, copies):
+    _run([0, 1, 2, 8, 40], copies, width, cap)
 
 
 def test_long_tables_of_many_terms_keep_to_the_chunk_forms():
