@@ -17,10 +17,11 @@
 // whose bytes complete the receiver's mbarrier themselves: a store followed by an arrive
 // with cluster-scope release cost 1,500-1,900 clocks a step.  Buffers alternate between two
 // slots: a neighbour sends its step-s columns only after it has read its own step-s buffers, and
-// this warp writes those buffers again only after receiving them, so two slots suffice.  One cluster barrier per sweep decides
-// convergence.  A warp whose wait gives up leaves the sweep, sends nothing more and says so at
-// that barrier: the whole cluster then stops and the sector's info word is -TNB_ETIMEOUT.  (Its
-// vote, behind the loads of the received columns, takes 1 % of the launch; before them 5 %.)
+// this warp writes those buffers again only after receiving them, so two slots suffice.  One
+// cluster barrier per sweep decides convergence.  A warp whose wait gives up leaves the sweep,
+// sends nothing more and says so at that barrier: the whole cluster then stops and the
+// sector's info word is -TNB_ETIMEOUT.  (Its vote, behind the loads of the received columns,
+// takes 1 % of the launch; before them 5 %.)
 //
 // Measured on B200 (the whole launch, before: block_svd_kernel): ten SU(2) sectors up to 116
 // x 116, 2.4 ms (16.5); two 128 x 128 sectors, 2.7 ms (18.9); sectors up to 49 x 49, 0.68
